@@ -219,7 +219,8 @@ int upload_constants() {
   int (*const up[])(const ConstTables &) = {upload_tables_cart_f64,    upload_tables_cart_f32,
                                             upload_tables_curv_f64,    upload_tables_curv_f32,
                                             upload_tables_generic_f64, upload_tables_generic_f32,
-                                            upload_tables_batch_f64,   upload_tables_batch_f32};
+                                            upload_tables_batch_f64,   upload_tables_batch_f32,
+                                            upload_tables_point_f64,   upload_tables_point_f32};
   for (auto f : up) {
     const int e = f(t);
     if (e != 0) return fail(WQL3D_ECUDA, std::string("stage constants: ") + cudaGetErrorString((cudaError_t)e));
@@ -1008,12 +1009,23 @@ int setup_block(wql3d_domain *d, int bi) {
   return WQL3D_OK;
 }
 
+// whether full stages of block bi run the two-role point kernels
+template <typename T>
+bool point_path(wql3d_domain *d, int bi) {
+  const Blk<T> &b = blk<T>(d, bi);
+  return !tuning().generic && !b.mms && b.fd == WQL3D_FD_TRADITIONAL6 && point_stage_ok(b, d->hb[bi].mesh);
+}
+
 template <typename T>
 void launch_stage(wql3d_domain *d, int bi, const StageArgs &a, bool fused = false) {
   Blk<T> &b = blk<T>(d, bi);
   const int mesh = d->hb[bi].mesh;
   StageCtx c{d->stream, d->response, &d->launches, d->side, d->fork, d->join};
   const bool special = tuning().generic || b.mms || b.fd != WQL3D_FD_TRADITIONAL6;
+  if (a.flags == F_ALL && point_path<T>(d, bi)) {
+    launch_point_stage<T>(b, mesh, c, a);
+    return;
+  }
   if (fused && mesh == WQL3D_MESH_CARTESIAN && a.flags == F_ALL && !special)
     launch_cart_stage<T>(b, c, a);
   else if (mesh == WQL3D_MESH_CURVILINEAR && b.G && !special)

@@ -44,6 +44,7 @@ struct Tuning {
   int fused_minb = 0; // k_curv_fused resident 128-thread blocks per SM: 3 (default), 2 or 4 in FP64; 4 (default), 5 or 6 in FP32
   int mvpf = -1;      // k_curv_fused: L2 prefetch of the memory variables on entry (-1: FP32 only)
   int overlap = 1;    // Cartesian stage: shell on the side stream, concurrent with the interior
+  int point = 1;      // separable Cartesian stages through the point kernels (0 when WQL3D_TMA is set: the tile kernel)
   int tma = 0;        // Cartesian interior: 1 = planes filled by TMA box loads (default: cp.async, measured faster);
                       // 2 = TMA waits with no copies issued (test of the bounded waits and the stall status)
 };
@@ -55,7 +56,10 @@ inline Tuning tuning() {
     if (const char *e = getenv("WQL3D_FUSED_MINB")) r.fused_minb = atoi(e);
     if (const char *e = getenv("WQL3D_MV_PREFETCH")) r.mvpf = atoi(e);
     if (const char *e = getenv("WQL3D_SHELL_OVERLAP")) r.overlap = atoi(e);
-    if (const char *e = getenv("WQL3D_TMA")) r.tma = atoi(e);
+    if (const char *e = getenv("WQL3D_TMA")) {
+      r.tma = atoi(e);
+      r.point = 0;
+    }
     if (const char *e = getenv("WQL3D_KERNEL")) {
       r.generic = strcmp(e, "generic") == 0;
       if (strcmp(e, "curv_generic_update") == 0) r.lean = 0;
@@ -83,6 +87,11 @@ void launch_cart_stage(Blk<T> &b, const StageCtx &c, const StageArgs &a);
 // curvilinear split stage: derivative pass, memory variables, face SATs, point update
 template <typename T>
 void launch_curv_stage(Blk<T> &b, const StageCtx &c, const StageArgs &a);
+// full stage (flags == F_ALL) through the two-role point kernels, both meshes
+template <typename T>
+void launch_point_stage(Blk<T> &b, int mesh, const StageCtx &c, const StageArgs &a);
+template <typename T>
+bool point_stage_ok(const Blk<T> &b, int mesh);
 // true when the block's full curvilinear stages run k_curv_fused (which can
 // record the adjoint's derivative terms, StageArgs::rec)
 template <typename T>
@@ -95,6 +104,8 @@ int upload_tables_cart_f64(const ConstTables &t);
 int upload_tables_cart_f32(const ConstTables &t);
 int upload_tables_curv_f64(const ConstTables &t);
 int upload_tables_curv_f32(const ConstTables &t);
+int upload_tables_point_f64(const ConstTables &t);
+int upload_tables_point_f32(const ConstTables &t);
 int upload_tables_generic_f64(const ConstTables &t);
 int upload_tables_generic_f32(const ConstTables &t);
 
