@@ -140,6 +140,9 @@ struct HostBlock {
   int nrec = 0;
   int nsrc = 0;
   int iface_side[2] = {0, 0};
+  // curvilinear blocks: the flux arrays of the current field buffer belong to
+  // the fields it holds (a stage of the point kernels left them there)
+  bool flux_ok = false;
 };
 
 struct wql3d_domain {
@@ -1013,7 +1016,18 @@ int setup_block(wql3d_domain *d, int bi) {
 template <typename T>
 bool point_path(wql3d_domain *d, int bi) {
   const Blk<T> &b = blk<T>(d, bi);
-  return !tuning().generic && !b.mms && b.fd == WQL3D_FD_TRADITIONAL6 && point_stage_ok(b, d->hb[bi].mesh);
+  return !tuning().generic && !b.mms && b.fd == WQL3D_FD_TRADITIONAL6 &&
+         point_stage_ok(b, d->hb[bi].mesh);
+}
+
+// the flux arrays of a curvilinear block on the point path, made current
+template <typename T>
+void ensure_fluxes(wql3d_domain *d, int bi) {
+  if (d->hb[bi].mesh != WQL3D_MESH_CURVILINEAR || d->hb[bi].flux_ok || !point_path<T>(d, bi)) return;
+  const Blk<T> &b = blk<T>(d, bi);
+  StageCtx c{d->stream, d->response, &d->launches};
+  launch_fluxes<T>(b, c, d->cur, b.open_lo[2] ? 1 - NB : 1, b.open_hi[2] ? b.nz + NB : b.nz);
+  d->hb[bi].flux_ok = true;
 }
 
 template <typename T>
@@ -1023,9 +1037,12 @@ void launch_stage(wql3d_domain *d, int bi, const StageArgs &a, bool fused = fals
   StageCtx c{d->stream, d->response, &d->launches, d->side, d->fork, d->join};
   const bool special = tuning().generic || b.mms || b.fd != WQL3D_FD_TRADITIONAL6;
   if (a.flags == F_ALL && point_path<T>(d, bi)) {
+    ensure_fluxes<T>(d, bi);
     launch_point_stage<T>(b, mesh, c, a);
+    d->hb[bi].flux_ok = mesh == WQL3D_MESH_CURVILINEAR;
     return;
   }
+  if (a.flags & F_UPDATE) d->hb[bi].flux_ok = false;
   if (fused && mesh == WQL3D_MESH_CARTESIAN && a.flags == F_ALL && !special)
     launch_cart_stage<T>(b, c, a);
   else if (mesh == WQL3D_MESH_CURVILINEAR && b.G && !special)
@@ -1085,6 +1102,7 @@ int run_steps(wql3d_domain *d, double dt, int nsteps, int w_stride) {
   // CUDA graph of two steps (five stages each, so the field-buffer parity
   // returns to its start) replayed nsteps/2 times
   int pairs = nsteps / 2;
+  for (int i = 0; i < d->nblocks; ++i) ensure_fluxes<T>(d, i);   // outside the captured steps
   if (pairs > 0) {
     if (!d->graph || d->g_dt != dt || d->g_w != w_stride || d->g_cur != d->cur) {
       if (d->graph) { cudaGraphExecDestroy(d->graph); d->graph = nullptr; }
@@ -1181,6 +1199,13 @@ int halo_launch(wql3d_domain *d, Blk<T> &b, int kind, int unpack) {
   const long long n = (long long)2 * ncomp * 3 * b.nx * b.ny;
   k_halo<T><<<(unsigned)((n + 255) / 256), 256, 0, d->stream>>>(b, buf, a0, n0, a1, ncomp, unpack);
   d->launches++;
+  if (unpack && kind != WQL3D_HALO_FIELDS) d->hb[0].flux_ok = false;
+  if (unpack && kind == WQL3D_HALO_FIELDS && d->hb[0].flux_ok) {
+    // the fluxes of the ghost planes just received
+    StageCtx c{d->stream, d->response, &d->launches};
+    if (b.open_lo[2]) launch_fluxes<T>(b, c, d->cur, 1 - NB, 0);
+    if (b.open_hi[2]) launch_fluxes<T>(b, c, d->cur, b.nz + 1, b.nz + NB);
+  }
   CK(cudaGetLastError());
   return WQL3D_OK;
 }
@@ -1326,6 +1351,7 @@ int wql3d_domain_destroy(wql3d_domain *d) {
 int wql3d_set_fields(wql3d_domain *d, int bi, const double *F, int32_t host_nb) {
   DOM_CHECK(d, bi);
   if (!F || host_nb < 0) return fail(WQL3D_EINVAL, "fields");
+  d->hb[bi].flux_ok = false;
   int rc = d->fp32 ? put_array<float>(d, d->hb[bi], d->cur ? d->bf[bi].F1 : d->bf[bi].F0, 9, F, host_nb)
                    : put_array<double>(d, d->hb[bi], d->cur ? d->bd[bi].F1 : d->bd[bi].F0, 9, F, host_nb);
   if (rc) return rc;
@@ -1659,6 +1685,7 @@ int wql3d_enforce_bound_iface_conditions(wql3d_domain *d, int stage) {
 int wql3d_update_fields(wql3d_domain *d, double dt) {
   if (!d) return fail(WQL3D_EINVAL, "null domain");
   for (int i = 0; i < d->nblocks; ++i) {
+    d->hb[i].flux_ok = false;
     if (d->fp32) {
       Blk<float> &b = d->bf[i];
       dim3 th(32, 4, 2), gr((b.nx + 31) / 32, (b.ny + 3) / 4, (b.nz + 1) / 2);
@@ -1888,6 +1915,7 @@ int wql3d_adjoint_step(wql3d_domain *d, int n, double dt) {
   }
   // leave the domain's fields at F^(0) = F_n
   d->cur = cur0;
+  d->hb[0].flux_ok = false;
   CK(cudaMemcpyAsync(d->cur ? b.F1 : b.F0, A.S[0], bytes, cudaMemcpyDeviceToDevice, d->stream));
   // reversed stages 5..1
   for (int s = 5; s >= 1; --s) {
@@ -2001,6 +2029,7 @@ int wql3d_load_fields(wql3d_domain *d, int bi, const double *dev_src) {
   DOM_CHECK(d, bi);
   if (d->fp32 || !dev_src) return fail(WQL3D_EINVAL, "FP64 domain and a device array");
   const Blk<double> &b = d->bd[bi];
+  d->hb[bi].flux_ok = false;
   CK(cudaMemcpyAsync(d->cur ? b.F1 : b.F0, dev_src, sizeof(double) * 9 * (size_t)b.vol, cudaMemcpyDeviceToDevice,
                      d->stream));
   return WQL3D_OK;

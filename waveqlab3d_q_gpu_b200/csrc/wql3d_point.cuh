@@ -276,6 +276,12 @@ __device__ __forceinline__ void axis_finish(const Blk<T> &b, const StageArgs &a,
       T *__restrict__ DQp = b.DQ[s] + q;
       const T d = slab_damp<AX>(b, s, i);
       const T A = (T)a.A, Bdt = (T)a.Bdt;
+      if constexpr (ROLE == ROLE_V && MESH == MESH_CURV) {
+        // the auxiliary velocities themselves: k_pml_velocity
+#pragma unroll
+        for (int c = 0; c < 3; ++c) df[c] = df[c] - d * Qp[c * PV] * irho;
+        return;
+      }
       T Q[NC], DQ[NC];
 #pragma unroll
       for (int c = 0; c < NC; ++c) {
@@ -404,6 +410,21 @@ __device__ __forceinline__ void memory_component(const Blk<T> &b, const StageArg
   asm volatile("" ::: "memory");
 }
 
+// contravariant stress fluxes G[3 a + c] = J sum_r X_r,a sigma_rc of one
+// point (f: stresses xx yy zz xy xz yz)
+template <typename T>
+__device__ __forceinline__ void store_fluxes(const Blk<T> &b, T *__restrict__ G, unsigned o, const T f[6]) {
+  const long long V = b.vol;
+  const T J = at(b.J, o);
+#pragma unroll
+  for (int ax = 0; ax < 3; ++ax) {
+    const T x0 = J * at(b.met + ax * V, o), x1 = J * at(b.met + (3 + ax) * V, o), x2 = J * at(b.met + (6 + ax) * V, o);
+    (G + (3 * ax) * V)[o] = x0 * f[0] + x1 * f[3] + x2 * f[4];
+    (G + (3 * ax + 1) * V)[o] = x0 * f[3] + x1 * f[1] + x2 * f[5];
+    (G + (3 * ax + 2) * V)[o] = x0 * f[4] + x1 * f[5] + x2 * f[2];
+  }
+}
+
 // one point of a full stage (flags F_ALL), velocity half
 template <typename T, int MESH, bool PML>
 __device__ __forceinline__ void point_v(const Blk<T> &b, const StageArgs &a, bool inner, int x, int y, int z) {
@@ -519,6 +540,7 @@ __device__ __forceinline__ void point_s(const Blk<T> &b, const StageArgs &a, boo
 #pragma unroll
   for (int c = 0; c < 6; ++c) f[c] = at(F + (3 + c) * V, o);
   role_store<T, ROLE_S>(b, a, o, df, f);
+  if constexpr (MESH == MESH_CURV) store_fluxes<T>(b, b.G + (a.cur ? 0 : 9 * V), o, f);
 }
 
 // Work map of a block, in warps: rows are taken two at a time (a row pair).
@@ -608,6 +630,114 @@ __global__ void __launch_bounds__(128, MINB) k_point(const __grid_constant__ Blk
   const int t = (blockIdx.x >> 1) * 128 + threadIdx.x;
   if (FLAT ? !flat_index(b, t, x, y, z) : !warp_point(b, m, t >> 5, t & 31, x, y, z)) return;
   run_role<T, MESH, RESP, PML>(b, a, blockIdx.x & 1 ? ROLE_S : ROLE_V, x, y, z);
+}
+
+// The contravariant fluxes of the fields F on planes z0 .. z1 (ghost planes
+// of open faces included), where no stage has left them: fields set by the
+// caller, restored or updated in place
+template <typename T>
+__global__ void __launch_bounds__(128) k_fluxes(Blk<T> b, int cur, int z0, int z1) {
+  const long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const long long plane = (long long)b.nx * b.ny;
+  if (j >= plane * (z1 - z0 + 1)) return;
+  const int z = z0 + (int)(j / plane);
+  const int r = (int)(j % plane), y = r / b.nx + 1, x = r % b.nx + 1;
+  const unsigned o = (unsigned)pidx(b, x, y, z);
+  const T *F = cur ? b.F1 : b.F0;
+  T f[6];
+#pragma unroll
+  for (int c = 0; c < 6; ++c) f[c] = (F + (3 + c) * b.vol)[o];
+  store_fluxes<T>(b, b.G + (cur ? 9 * b.vol : 0), o, f);
+}
+
+// Auxiliary velocities (Q, DQ 0-2) of every PML slab of a curvilinear block,
+// src/RHS_Interior.f90:1913-2265: the source on the slab of axis A is the
+// flux divergence of metric row A alone, D_a(J X_A,a sigma_Ac) / J, which the
+// summed fluxes of the velocity half do not hold, so it is gathered here, for
+// slab points only.  Runs after the velocity half, which damps with the old Q.
+// One thread per slab point, `first` the CTA offsets of the six faces.
+struct SlabCtas {
+  int first[7];
+};
+template <typename T>
+__global__ void __launch_bounds__(128, sizeof(T) == 8 ? 4 : 8) k_pml_velocity(const __grid_constant__ Blk<T> b,
+                                                                            const __grid_constant__ StageArgs a,
+                                                                            SlabCtas m) {
+  int f = 0;
+#pragma unroll
+  for (int g = 1; g < 6; ++g)
+    if ((int)blockIdx.x >= m.first[g]) f = g;
+  const long long k = (long long)(blockIdx.x - m.first[f]) * 128 + threadIdx.x;
+  const long long PV = b.pvol[f];
+  if (k >= PV) return;
+  const int *B = b.pb[f];
+  const int wx = B[1] - B[0] + 1, wy = B[3] - B[2] + 1;
+  const int r = (int)(k / wx), x = B[0] + (int)(k - (long long)r * wx), z = B[4] + r / wy, y = B[2] + r % wy;
+  const unsigned o = (unsigned)pidx(b, x, y, z);
+  const long long V = b.vol;
+  const T *__restrict__ F = a.cur ? b.F1 : b.F0;
+  T *__restrict__ Qp = b.Q[f] + k;
+  T *__restrict__ DQp = b.DQ[f] + k;
+  const int AX = f >> 1;
+  const T *__restrict__ s0 = F + (AX == 0 ? 3 : 5 + AX) * V;   // sigma_A0
+  const T *__restrict__ s1 = F + (AX == 1 ? 4 : 6 + AX) * V;   // sigma_A1
+  const T *__restrict__ s2 = F + (AX == 2 ? 5 : 7 + AX) * V;   // sigma_A2
+  T Q[3], DQ[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    Q[c] = Qp[c * PV];
+    DQ[c] = DQp[c * PV];
+  }
+  const int pos[3] = {x, y, z}, nn[3] = {b.nx, b.ny, b.nz}, st[3] = {1, (int)b.sy, (int)b.sz};
+  const T ih[3] = {b.ihq, b.ihr, b.ihs};
+  T S[3] = {0, 0, 0};
+#pragma unroll
+  for (int ax = 0; ax < 3; ++ax) {
+    const T *__restrict__ X = b.met + (long long)(3 * AX + ax) * V;
+    const int i = pos[ax], n = nn[ax];
+    T d[3] = {0, 0, 0};
+    if (central_row(b, ax, i, n)) {
+      T w[6], t0[6], t1[6], t2[6];
+      load6(b.J, o, st[ax], w);
+      load6(X, o, st[ax], t0);
+#pragma unroll
+      for (int q = 0; q < 6; ++q) w[q] *= t0[q];
+      load6(s0, o, st[ax], t0);
+      load6(s1, o, st[ax], t1);
+      load6(s2, o, st[ax], t2);
+#pragma unroll
+      for (int q = 0; q < 6; ++q) { t0[q] *= w[q]; t1[q] *= w[q]; t2[q] *= w[q]; }
+      d[0] = central(t0); d[1] = central(t1); d[2] = central(t2);
+    } else {
+      const int row = i <= 6 ? i - 1 : 6 + (n - i);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const T c = (T)__ldg(b.rowc + row * 8 + q);
+        if (c != (T)0) {
+          const unsigned p = o + (unsigned)(__ldg(b.rowo + row * 8 + q) * st[ax]);
+          const T w = c * (at(b.J, p) * at(X, p));
+          d[0] = d[0] + w * at(s0, p);
+          d[1] = d[1] + w * at(s1, p);
+          d[2] = d[2] + w * at(s2, p);
+        }
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) S[c] = S[c] + ih[ax] * d[c];
+  }
+  const T iJ = (T)1 / at(b.J, o);
+  const T d = AX == 0 ? slab_damp<0>(b, f, x) : AX == 1 ? slab_damp<1>(b, f, y) : slab_damp<2>(b, f, z);
+  const bool face = (f & 1) ? pos[AX] == nn[AX] : pos[AX] == 1;
+  const T *__restrict__ fq = b.fdq[f];
+  const int fn = b.foff[f + 1] - b.foff[f];
+  const int fk = AX == 0 ? (y - 1) + b.ny * (z - 1) : AX == 1 ? (x - 1) + b.nx * (z - 1) : (x - 1) + b.nx * (y - 1);
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    T q = (T)a.A * DQ[c] + S[c] * iJ - (d + (T)1) * Q[c];
+    if (face && fq) q = q - fq[c * fn + fk];
+    DQp[c * PV] = q;
+    Qp[c * PV] = Q[c] + (T)a.Bdt * q;
+  }
 }
 
 }  // namespace wql3d

@@ -90,6 +90,10 @@ void launch_curv_stage(Blk<T> &b, const StageCtx &c, const StageArgs &a);
 // full stage (flags == F_ALL) through the two-role point kernels, both meshes
 template <typename T>
 void launch_point_stage(Blk<T> &b, int mesh, const StageCtx &c, const StageArgs &a);
+// contravariant stress fluxes of buffer `cur` on planes z0 .. z1 (curvilinear
+// blocks; the point kernels read them and leave the next stage's)
+template <typename T>
+void launch_fluxes(const Blk<T> &b, const StageCtx &c, int cur, int z0, int z1);
 template <typename T>
 bool point_stage_ok(const Blk<T> &b, int mesh);
 // true when the block's full curvilinear stages run k_curv_fused (which can
