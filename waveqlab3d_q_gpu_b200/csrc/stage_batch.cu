@@ -5,11 +5,14 @@
 // descriptor in shared memory before running the same tile / point bodies as
 // the per-domain kernels (interior_split_tile, point_update, sample_block).
 //
-// Work lists: every CTA belongs to one shot.  The interior launch covers the
-// shots' 32 x 4 x zchunk tiles, the shell launch their near-boundary points
-// in chunks of 128 (each shot's chunk count rounded up, so no CTA straddles
-// two shots); a prefix array over the class's shots maps a CTA to its shot.
+// Work lists: every CTA belongs to one shot.  Separable blocks run the two
+// roles of the point kernels (k_batch_point, pairs of CTAs over 128
+// consecutive points); the others an interior launch over their 32 x 4 x
+// zchunk tiles and a shell launch over their near-boundary points in chunks of
+// 128 (each shot's chunk count rounded up, so no CTA straddles two shots).  A
+// prefix array over the class's shots maps a CTA to its shot.
 #include "wql3d_batch.cuh"
+#include "wql3d_point.cuh"
 
 namespace wql3d {
 
@@ -55,7 +58,29 @@ __global__ void __launch_bounds__(256, 2) k_batch_interior(BatchClass<T> C, Stag
   interior_split_tile<T, RESP, 4>(sb, la, zchunk, bx, by, bz, smraw);
 }
 
-template <typename T, int RESP, bool SEP>
+// Both roles of every separable shot: 186 -> 162 ms per 24 FP32 steps on eight
+// elastic and Q4 shots of 64^3 to 128^3 points, against interior tiles beside a
+// shell launch.  MINB is tuned over the batch's first steps.
+template <typename T, int RESP, int MINB>
+__global__ void __launch_bounds__(128, MINB) k_batch_point(BatchClass<T> C, const __grid_constant__ StageArgs a) {
+  __shared__ __align__(16) Blk<T> sb;
+  __shared__ int s_shot, s_local;
+  if (threadIdx.x == 0) {
+    const int k = owner(C.tile_prefix, C.nshots, blockIdx.x);
+    s_shot = C.shots[k];
+    s_local = blockIdx.x - C.tile_prefix[k];
+  }
+  __syncthreads();
+  stage_blk<T>(C.blks + s_shot, &sb);
+  __syncthreads();
+  StageArgs la = a;
+  la.time = C.times[s_shot];
+  int x, y, z;
+  if (!flat_index(sb, (s_local >> 1) * 128 + (int)threadIdx.x, x, y, z)) return;
+  run_role<T, MESH_CART, RESP, false>(sb, la, s_local & 1 ? ROLE_S : ROLE_V, x, y, z);
+}
+
+template <typename T, int RESP>
 __global__ void __launch_bounds__(128, 3) k_batch_shell(BatchClass<T> C, StageArgs a) {
   __shared__ __align__(16) Blk<T> sb;
   __shared__ int s_shot, s_local;
@@ -73,7 +98,7 @@ __global__ void __launch_bounds__(128, 3) k_batch_shell(BatchClass<T> C, StageAr
   shell_decode(sb, (int)idx, x, y, z);
   StageArgs la = a;
   la.time = C.times[s_shot];
-  point_update<T, MESH_CART, RESP, SEP, false, true>(sb, la, x, y, z);
+  point_update<T, MESH_CART, RESP, false, false, true>(sb, la, x, y, z);
 }
 
 // stage-1 station samples of every shot: one CTA per shot
@@ -99,8 +124,23 @@ __global__ void k_batch_advance(DevTime *const *times, int n, double dt) {
 
 // interior tiles (part 0) or near-boundary shell (part 1) of one class
 template <typename T, int RESP>
-void launch_class(const BatchClass<T> &C, const StageArgs &a, int zchunk, cudaStream_t s, int part,
+void launch_class(const BatchClass<T> &C, const StageArgs &a, int zchunk, int minb, cudaStream_t s, int part,
                   int64_t *launches) {
+  if (C.sep) {
+    if (part != 0 || C.tiles <= 0) return;
+    StageArgs la = a;
+    la.pf = sizeof(T) == 4 ? 1 : 0;
+    switch (minb) {
+      case 3: k_batch_point<T, RESP, 3><<<C.tiles, 128, 0, s>>>(C, la); break;
+      case 4: k_batch_point<T, RESP, 4><<<C.tiles, 128, 0, s>>>(C, la); break;
+      case 5: k_batch_point<T, RESP, 5><<<C.tiles, 128, 0, s>>>(C, la); break;
+      case 7: k_batch_point<T, RESP, 7><<<C.tiles, 128, 0, s>>>(C, la); break;
+      case 8: k_batch_point<T, RESP, 8><<<C.tiles, 128, 0, s>>>(C, la); break;
+      default: k_batch_point<T, RESP, 6><<<C.tiles, 128, 0, s>>>(C, la); break;
+    }
+    ++*launches;
+    return;
+  }
   if (part == 0 && C.tiles > 0) {
     const size_t sm = SplitSmem<T, 4>::bytes;
     cudaFuncSetAttribute(k_batch_interior<T, RESP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
@@ -108,23 +148,22 @@ void launch_class(const BatchClass<T> &C, const StageArgs &a, int zchunk, cudaSt
     ++*launches;
   }
   if (part == 1 && C.shell_ctas > 0) {
-    if (C.sep) k_batch_shell<T, RESP, true><<<C.shell_ctas, 128, 0, s>>>(C, a);
-    else k_batch_shell<T, RESP, false><<<C.shell_ctas, 128, 0, s>>>(C, a);
+    k_batch_shell<T, RESP><<<C.shell_ctas, 128, 0, s>>>(C, a);
     ++*launches;
   }
 }
 
 template <typename T>
-void launch_part(const BatchClass<T> *classes, int ncls, const StageArgs &a, int zchunk, cudaStream_t s, int part,
-                 int64_t *launches) {
+void launch_part(const BatchClass<T> *classes, int ncls, const StageArgs &a, int zchunk, int minb, cudaStream_t s,
+                 int part, int64_t *launches) {
   for (int c = 0; c < ncls; ++c) {
     const BatchClass<T> &C = classes[c];
     if (C.nshots == 0) continue;
     switch (C.resp) {
-      case RESP_EL: launch_class<T, RESP_EL>(C, a, zchunk, s, part, launches); break;
-      case RESP_Q4: launch_class<T, RESP_Q4>(C, a, zchunk, s, part, launches); break;
-      case RESP_Q8: launch_class<T, RESP_Q8>(C, a, zchunk, s, part, launches); break;
-      default: launch_class<T, RESP_FQ8>(C, a, zchunk, s, part, launches); break;
+      case RESP_EL: launch_class<T, RESP_EL>(C, a, zchunk, minb, s, part, launches); break;
+      case RESP_Q4: launch_class<T, RESP_Q4>(C, a, zchunk, minb, s, part, launches); break;
+      case RESP_Q8: launch_class<T, RESP_Q8>(C, a, zchunk, minb, s, part, launches); break;
+      default: launch_class<T, RESP_FQ8>(C, a, zchunk, minb, s, part, launches); break;
     }
   }
 }
@@ -132,21 +171,21 @@ void launch_part(const BatchClass<T> *classes, int ncls, const StageArgs &a, int
 }  // namespace
 
 template <typename T>
-void launch_batch_stage(const BatchClass<T> *classes, int ncls, const StageArgs &a, int zchunk, cudaStream_t s,
-                        cudaStream_t side, cudaEvent_t fork, cudaEvent_t join, int64_t *launches) {
+void launch_batch_stage(const BatchClass<T> *classes, int ncls, const StageArgs &a, int zchunk, int minb,
+                        cudaStream_t s, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join, int64_t *launches) {
   if (side) {
     // every class's shell on the side stream, next to the interior tiles
     // (disjoint points of independent shots)
     cudaEventRecord(fork, s);
     cudaStreamWaitEvent(side, fork, 0);
-    launch_part<T>(classes, ncls, a, zchunk, side, 1, launches);
+    launch_part<T>(classes, ncls, a, zchunk, minb, side, 1, launches);
     cudaEventRecord(join, side);
-    launch_part<T>(classes, ncls, a, zchunk, s, 0, launches);
+    launch_part<T>(classes, ncls, a, zchunk, minb, s, 0, launches);
     cudaStreamWaitEvent(s, join, 0);
     return;
   }
-  launch_part<T>(classes, ncls, a, zchunk, s, 0, launches);
-  launch_part<T>(classes, ncls, a, zchunk, s, 1, launches);
+  launch_part<T>(classes, ncls, a, zchunk, minb, s, 0, launches);
+  launch_part<T>(classes, ncls, a, zchunk, minb, s, 1, launches);
 }
 
 template <typename T>
@@ -163,7 +202,7 @@ void launch_batch_advance(DevTime *const *times, int nshots, double dt, cudaStre
 }
 
 template void launch_batch_stage<WQL3D_REAL>(const BatchClass<WQL3D_REAL> *, int, const StageArgs &, int,
-                                             cudaStream_t, cudaStream_t, cudaEvent_t, cudaEvent_t, int64_t *);
+                                             int, cudaStream_t, cudaStream_t, cudaEvent_t, cudaEvent_t, int64_t *);
 template void launch_batch_sample<WQL3D_REAL>(const Blk<WQL3D_REAL> *, DevTime *const *, int, int, int,
                                               cudaStream_t, int64_t *);
 template void launch_batch_advance<WQL3D_REAL>(DevTime *const *, int, double, cudaStream_t, int64_t *);

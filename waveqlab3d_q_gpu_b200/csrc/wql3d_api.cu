@@ -2139,11 +2139,13 @@ struct wql3d_batch {
     int tiles = 0, shell_ctas = 0;
   } cls[8];
   int zchunk = 12;
+  int minb = 6;                   // resident CTAs of the point kernels
+  bool points = false;            // every class runs the point kernels: minb is tuned, else zchunk
   int tuned = 0;
   int cur = 0;
   cudaGraphExec_t graph = nullptr;
   double g_dt = 0.0;
-  int g_w = -1, g_cur = -1, g_z = -1;
+  int g_w = -1, g_cur = -1, g_z = -1, g_minb = -1;
   int64_t g_launches = 0, launches = 0;
   std::vector<std::pair<int, float>> tune_log;   // (zchunk, ms per step) of the tuning steps
 };
@@ -2159,7 +2161,8 @@ int batch_tiles(wql3d_batch *bt) {
       const wql3d_domain *d = bt->doms[(size_t)c.shots[i]];
       const int *lo = bt->fp32 ? d->bf[0].lo : d->bd[0].lo, *hi = bt->fp32 ? d->bf[0].hi : d->bd[0].hi;
       const int nxi = hi[0] - lo[0] + 1, nyi = hi[1] - lo[1] + 1, nzi = hi[2] - lo[2] + 1;
-      const int t = (nxi > 0 && nyi > 0 && nzi > 0)
+      const long long np = (long long)d->hb[0].nq * d->hb[0].nr * d->hb[0].ns;
+      const int t = c.sep ? 2 * (int)((np + 127) / 128) : (nxi > 0 && nyi > 0 && nzi > 0)
                         ? ((nxi + 31) / 32) * ((nyi + 3) / 4) * ((nzi + bt->zchunk - 1) / bt->zchunk) : 0;
       pre[i + 1] = pre[i] + t;
     }
@@ -2198,7 +2201,8 @@ void batch_enqueue_step(wql3d_batch *bt, double dt, int w_stride) {
     a.Bdt = kRkB[st - 1] * dt;
     a.dt = dt;
     a.time = nullptr;
-    launch_batch_stage<T>(cl, ncl, a, bt->zchunk, bt->stream, tuning().overlap ? bt->side : nullptr, bt->fork,
+    launch_batch_stage<T>(cl, ncl, a, bt->zchunk, bt->minb, bt->stream,
+                          tuning().overlap && !bt->points ? bt->side : nullptr, bt->fork,
                           bt->join, &bt->launches);
     bt->cur ^= 1;
   }
@@ -2207,15 +2211,18 @@ void batch_enqueue_step(wql3d_batch *bt, double dt, int w_stride) {
 
 template <typename T>
 int batch_run(wql3d_batch *bt, double dt, int nsteps, int w_stride) {
-  // project-written tile autotuner: the first steps of the first run each try
-  // one z-chunk length of the interior tiles (the arithmetic of a point does
-  // not depend on it), timed with events; the fastest is kept
+  // project-written autotuner: the first steps of the first run each try one
+  // launch shape (the arithmetic of a point does not depend on it), timed with
+  // events; the fastest is kept: the resident CTAs of the point kernels, or the
+  // z-chunk length of the interior tiles where a shot needs those
   if (!bt->tuned) {
-    const int cand[6] = {4, 8, 12, 16, 24, 32};
+    const int zcand[6] = {4, 8, 12, 16, 24, 32}, pcand[6] = {3, 4, 5, 6, 7, 8};
+    const int *cand = bt->points ? pcand : zcand;
+    int &shape = bt->points ? bt->minb : bt->zchunk;
     float best = 1e30f;
-    int bestz = bt->zchunk;
+    int bestz = shape;
     for (int i = 0; i < 6 && nsteps > 0; ++i) {
-      bt->zchunk = cand[i];
+      shape = cand[i];
       if (int rc = batch_tiles(bt)) return rc;
       cudaEvent_t e0, e1;
       CK(cudaEventCreate(&e0));
@@ -2232,14 +2239,15 @@ int batch_run(wql3d_batch *bt, double dt, int nsteps, int w_stride) {
       if (ms < best) { best = ms; bestz = cand[i]; }
       --nsteps;
     }
-    bt->zchunk = bestz;
+    shape = bestz;
     if (int rc = batch_tiles(bt)) return rc;
     bt->tuned = 1;
   }
   // CUDA graph of two steps of the whole batch, replayed
   const int pairs = nsteps / 2;
   if (pairs > 0) {
-    if (!bt->graph || bt->g_dt != dt || bt->g_w != w_stride || bt->g_cur != bt->cur || bt->g_z != bt->zchunk) {
+    if (!bt->graph || bt->g_dt != dt || bt->g_w != w_stride || bt->g_cur != bt->cur || bt->g_z != bt->zchunk ||
+        bt->g_minb != bt->minb) {
       if (bt->graph) { cudaGraphExecDestroy(bt->graph); bt->graph = nullptr; }
       const int cur0 = bt->cur;
       const int64_t l0 = bt->launches;
@@ -2255,6 +2263,7 @@ int batch_run(wql3d_batch *bt, double dt, int nsteps, int w_stride) {
       bt->g_w = w_stride;
       bt->g_cur = cur0;
       bt->g_z = bt->zchunk;
+      bt->g_minb = bt->minb;
       bt->g_launches = bt->launches - l0;
       bt->launches = l0;
     }
@@ -2337,6 +2346,8 @@ int wql3d_batch_create(wql3d_domain *const *domains, int32_t n, wql3d_batch **ou
     c.sep = sep ? 1 : 0;
     c.shots.push_back(i);
   }
+  bt->points = true;
+  for (const auto &c : bt->cls) bt->points = bt->points && (c.shots.empty() || c.sep);
   for (auto &c : bt->cls) {
     if (c.shots.empty()) continue;
     const size_t m = c.shots.size();
@@ -2381,7 +2392,7 @@ int wql3d_batch_run(wql3d_batch *bt, double dt, int32_t nsteps, int32_t w_stride
 
 int wql3d_batch_tuning(wql3d_batch *bt, int32_t *zchunk, int32_t *ntried, int32_t *zs, float *ms) {
   if (!bt) return fail(WQL3D_EINVAL, "null batch");
-  if (zchunk) *zchunk = bt->zchunk;
+  if (zchunk) *zchunk = bt->points ? bt->minb : bt->zchunk;
   if (ntried) *ntried = (int32_t)bt->tune_log.size();
   for (size_t i = 0; i < bt->tune_log.size(); ++i) {
     if (zs) zs[i] = bt->tune_log[i].first;

@@ -14,18 +14,19 @@ struct BatchClass {
   int resp, sep;
   int nshots;              // shots of this class
   const int *shots;        // their indices in the batch
-  const int *tile_prefix;  // interior CTAs: nshots + 1 offsets
-  const int *shell_prefix; // shell CTAs (128 points each): nshots + 1 offsets
+  const int *tile_prefix;  // CTAs of the point kernel (sep) or interior tiles: nshots + 1 offsets
+  const int *shell_prefix; // shell CTAs (128 points each; full-metric blocks): nshots + 1 offsets
   int tiles, shell_ctas;   // totals
   const Blk<T> *blks;      // every shot's block descriptor (device)
   DevTime *const *times;   // every shot's step time / sample counter (device)
 };
 
-// side != nullptr: the shells run on the side stream (fork / join events),
+// zchunk: planes of an interior tile; minb: resident CTAs the point kernels
+// are compiled for (3 to 8).  side != nullptr: the shells run on the side stream (fork / join events),
 // concurrently with the interior tiles
 template <typename T>
-void launch_batch_stage(const BatchClass<T> *classes, int ncls, const StageArgs &a, int zchunk, cudaStream_t s,
-                        cudaStream_t side, cudaEvent_t fork, cudaEvent_t join, int64_t *launches);
+void launch_batch_stage(const BatchClass<T> *classes, int ncls, const StageArgs &a, int zchunk, int minb,
+                        cudaStream_t s, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join, int64_t *launches);
 template <typename T>
 void launch_batch_sample(const Blk<T> *blks, DevTime *const *times, int nshots, int cur, int w_stride,
                          cudaStream_t s, int64_t *launches);

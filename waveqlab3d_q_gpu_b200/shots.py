@@ -76,7 +76,7 @@ class ShotBatch:
 
     mode 'batched' (default): one launch per kernel kind and RK stage for
     every shot (``wql3d_batch_*``: shot x tile work lists, the step pair in one
-    CUDA graph, interior tiles autotuned over the first steps).  mode
+    CUDA graph, the launch shape autotuned over the first steps).  mode
     'streams': each shot a domain on its own stream, its step graph replayed
     round-robin.  The shots share one time step (same spacing and rho_s_p, as
     :func:`random_shots` builds them)."""
@@ -122,7 +122,8 @@ class ShotBatch:
             done += k
 
     def tuning(self):
-        """(chosen z-chunk, [(candidate, ms per step), ...]) of the batch's tile autotuner."""
+        """(chosen launch shape, [(candidate, ms per step), ...]) of the batch's autotuner: CTAs per SM of the
+        point kernels, or the interior tiles' z-chunk where a shot needs those (wql3d_batch_tuning)."""
         import ctypes as C
         from . import _lib
         z, n = C.c_int32(), C.c_int32()
