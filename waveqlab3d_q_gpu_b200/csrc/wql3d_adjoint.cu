@@ -14,8 +14,15 @@ namespace {
 //   g_lambda += (R_xx + R_yy + R_zz) tr(grad v)
 //   g_mu     += 2 (R_xx v_x,x + R_yy v_y,y + R_zz v_z,z) + R_xy (v_x,y + v_y,x) + ...
 //   g_rho    += -1 / (rho^2 J) sum_f R_{v_f} (flux sum)_f
-__global__ void __launch_bounds__(128, 3) k_adj_pre(Blk<double> b, AdjBlk A, double Bdt, double As,
-                                                    const double *__restrict__ Sprev, const double *__restrict__ E) {
+// REC: the derivative terms E were recorded by the forward pass, and the
+// kernel is a stream of 67 words per point (80 registers, 6 resident CTAs); in
+// one kernel with the recomputing form it ran with that form's 168 registers
+// and 3 CTAs (99 us on 81 x 97 x 65 points, now 67; the stream alone is 41).
+template <bool REC>
+__global__ void __launch_bounds__(128, REC ? 5 : 3) k_adj_pre(const __grid_constant__ Blk<double> b,
+                                                              const __grid_constant__ AdjBlk A, double Bdt, double As,
+                                                              const double *__restrict__ Sprev,
+                                                              const double *__restrict__ E) {
   int x, y, z;
   if (!flat_point(b, x, y, z)) return;
   const long long p = pidx(b, x, y, z);
@@ -58,7 +65,7 @@ __global__ void __launch_bounds__(128, 3) k_adj_pre(Blk<double> b, AdjBlk A, dou
   // derivative terms of the stage input: recorded by the forward pass, or
   // recomputed (e: normal and shear strain rates, fs: stress-flux sums)
   double e[6], fs[3];
-  if (E) {
+  if constexpr (REC) {
 #pragma unroll
     for (int c = 0; c < 6; ++c) e[c] = E[c * V + p];
 #pragma unroll
@@ -134,19 +141,14 @@ __global__ void __launch_bounds__(128, 4) k_adj_stencil(Blk<double> b, AdjBlk A)
 // Face pass: the SAT term DF(p) -= pen * structure(bc(u(p))) of every face
 // point with a physical boundary condition, in the reference's face order:
 // Fbar(p) -= Jac^T R(p) and the material gradient by dual numbers at the
-// stage input.  Edge and corner points belong to several faces: atomics.
-__global__ void __launch_bounds__(128) k_adj_face(Blk<double> b, AdjBlk A, const double *__restrict__ Sprev,
-                                                 int f, int count) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= count) return;
+// stage input.  A point on several faces (edges, corners) is one thread's, face
+// after face, so that the sums have one order.
+__device__ __forceinline__ void adj_face_point(const Blk<double> &b, const AdjBlk &A, const double *__restrict__ Sprev,
+                                               int f, int x, int y, int z) {
   const int axis = f >> 1, plus = f & 1;
   const int d0 = axis == 0 ? b.ny : b.nx;
-  const int a1 = k / d0, a0 = k - a1 * d0;
-  const int fixed = plus ? (axis == 0 ? b.nx : axis == 1 ? b.ny : b.nz) : 1;
-  int x, y, z;
-  if (axis == 0) { x = fixed; y = a0 + 1; z = a1 + 1; }
-  else if (axis == 1) { x = a0 + 1; y = fixed; z = a1 + 1; }
-  else { x = a0 + 1; y = a1 + 1; z = fixed; }
+  const long long k = axis == 0 ? (y - 1) + (long long)b.ny * (z - 1)
+                                : axis == 1 ? (x - 1) + (long long)b.nx * (z - 1) : (x - 1) + (long long)b.nx * (y - 1);
   const long long p = pidx(b, x, y, z);
   const long long V = b.vol;
   const int type = b.bc[f];
@@ -182,7 +184,7 @@ __global__ void __launch_bounds__(128) k_adj_face(Blk<double> b, AdjBlk A, const
     double acc = 0.0;
 #pragma unroll
     for (int c = 0; c < 9; ++c) acc += out[c] * R[c];
-    atomicAdd(A.Fb + j * V + p, -acc);
+    A.Fb[j * V + p] -= acc;
   }
   // material derivatives at the stage input
   Dual u[9], ld3[3], md3[3], nd3[3];
@@ -197,16 +199,15 @@ __global__ void __launch_bounds__(128) k_adj_face(Blk<double> b, AdjBlk A, const
     double acc = 0.0;
 #pragma unroll
     for (int c = 0; c < 9; ++c) acc += out[c].b * R[c];
-    atomicAdd(A.g + prm * V + p, -acc);
+    A.g[prm * V + p] -= acc;
   }
 }
 
 // moment-tensor gradient of the sources at the stage time t: one block per
 // source over its delta support, gM[6 i + c] -= A_i(t) sum delta R_(3+c)
-__global__ void __launch_bounds__(256) k_adj_moment(Blk<double> b, AdjBlk A, double t) {
-  const int i = blockIdx.x;
+__device__ __forceinline__ void adj_moment_source(const Blk<double> &b, const AdjBlk &A, double t, int i,
+                                                  double red[6][128]) {
   const DevSource &s = b.src[i];
-  __shared__ double red[6][256];
   double acc[6] = {0, 0, 0, 0, 0, 0};
   if (s.near[0] >= 1) {
     const int hw = b.src_half, w = 2 * hw + 1;
@@ -237,6 +238,44 @@ __global__ void __launch_bounds__(256) k_adj_moment(Blk<double> b, AdjBlk A, dou
   if (threadIdx.x < 6) A.gM[6 * i + threadIdx.x] += red[threadIdx.x][0];
 }
 
+// Everything of a reversed stage that reads R beside the gather, in one
+// launch: the points of every face with a physical boundary condition (CTAs
+// first[f] .. first[f + 1] - 1 of face f), then one CTA per source.  As seven
+// launches of a few CTAs each these took 65 + 17 us of a 255 us stage on
+// 81 x 97 x 65 points, as one 45 us.
+struct FaceCtas {
+  int first[7];
+};
+__global__ void __launch_bounds__(128) k_adj_face(const __grid_constant__ Blk<double> b,
+                                                 const __grid_constant__ AdjBlk A, const double *__restrict__ Sprev,
+                                                 FaceCtas m, double t) {
+  __shared__ double red[6][128];
+  const int c = blockIdx.x;
+  if (c >= m.first[6]) {
+    adj_moment_source(b, A, t, c - m.first[6], red);
+    return;
+  }
+  int f = 0;
+#pragma unroll
+  for (int g = 1; g < 6; ++g)
+    if (c >= m.first[g]) f = g;
+  const int axis = f >> 1, d0 = axis == 0 ? b.ny : b.nx, d1 = axis == 2 ? b.ny : b.nz;
+  const int k = (c - m.first[f]) * 128 + threadIdx.x;
+  if (k >= d0 * d1) return;
+  const int nn[3] = {b.nx, b.ny, b.nz};
+  const int i1 = k / d0 + 1, i0 = k - (i1 - 1) * d0 + 1, fixed = (f & 1) ? nn[axis] : 1;
+  int pos[3];
+  pos[0] = axis == 0 ? fixed : i0;
+  pos[1] = axis == 1 ? fixed : axis == 0 ? i0 : i1;
+  pos[2] = axis == 2 ? fixed : i1;
+#pragma unroll 1
+  for (int g = 0; g < 6; ++g) {
+    if (b.bc[g] <= 0 || pos[g >> 1] != ((g & 1) ? nn[g >> 1] : 1)) continue;
+    if (g < f) return;   // that face's thread takes the point
+    adj_face_point(b, A, Sprev, g, pos[0], pos[1], pos[2]);
+  }
+}
+
 // receiver residuals of one sample into the velocity adjoint at the stations' nodes
 __global__ void k_adj_receivers(Blk<double> b, AdjBlk A) {
   for (int r = threadIdx.x; r < b.nrec; r += blockDim.x) {
@@ -250,26 +289,27 @@ __global__ void k_adj_receivers(Blk<double> b, AdjBlk A) {
 
 }  // namespace
 
-void adj_launch_stage(const Blk<double> &b, const AdjBlk &A, int stage, double Bdt, double A_s, cudaStream_t s,
-                      int64_t *launches) {
+void adj_launch_stage(const Blk<double> &b, const AdjBlk &A, int stage, double Bdt, double A_s, bool moment, double t,
+                      cudaStream_t s, int64_t *launches) {
   const long long npts = (long long)b.nx * b.ny * b.nz;
   const unsigned gr = (unsigned)((npts + 127) / 128);
-  k_adj_pre<<<gr, 128, 0, s>>>(b, A, Bdt, A_s, A.S[stage - 1], A.E[stage - 1]);
+  const double *S = A.S[stage - 1], *E = A.E[stage - 1];
+  if (E) k_adj_pre<true><<<gr, 128, 0, s>>>(b, A, Bdt, A_s, S, E);
+  else k_adj_pre<false><<<gr, 128, 0, s>>>(b, A, Bdt, A_s, S, E);
   ++*launches;
+  FaceCtas m;
+  m.first[0] = 0;
   for (int f = 0; f < 6; ++f) {
-    if (b.bc[f] <= 0) continue;
     const int axis = f >> 1;
     const int count = axis == 0 ? b.ny * b.nz : axis == 1 ? b.nx * b.nz : b.nx * b.ny;
-    k_adj_face<<<(count + 127) / 128, 128, 0, s>>>(b, A, A.S[stage - 1], f, count);
+    m.first[f + 1] = m.first[f] + (b.bc[f] > 0 ? (count + 127) / 128 : 0);
+  }
+  const int ctas = m.first[6] + (moment ? b.nsrc : 0);
+  if (ctas > 0) {
+    k_adj_face<<<ctas, 128, 0, s>>>(b, A, S, m, t);
     ++*launches;
   }
   k_adj_stencil<<<gr, 128, 0, s>>>(b, A);
-  ++*launches;
-}
-
-void adj_launch_moment(const Blk<double> &b, const AdjBlk &A, double t, cudaStream_t s, int64_t *launches) {
-  if (b.nsrc <= 0) return;
-  k_adj_moment<<<b.nsrc, 256, 0, s>>>(b, A, t);
   ++*launches;
 }
 

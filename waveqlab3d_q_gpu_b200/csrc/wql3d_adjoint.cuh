@@ -34,7 +34,7 @@ struct AdjBlk {
   double *g;              // material gradient: lambda, mu, rho (3 comps)
   double *gM;             // moment-tensor gradient, nsrc x 6 (mxx myy mzz mxy mxz myz)
   double *S[5];           // stage inputs F^(0..4) of the step being reversed (9 comps each)
-  const double *E[5];     // their derivative terms recorded by k_curv_fused (StageArgs::rec), or null
+  const double *E[5];     // their derivative terms recorded by the stage kernels (StageArgs::rec), or null
   const int *toff[3];     // transposed derivative rows per axis: [n][ADJ_TW] offsets
   const double *tc[3];    // ... and coefficients (0 pads)
   const double *res;      // receiver residuals of one sample, nrec x 3
@@ -85,9 +85,9 @@ __device__ void sat_term(int plus, const T u[9], T rho, T mu, T lam, const T l[3
 }
 
 // host launchers (wql3d_adjoint.cu)
-void adj_launch_stage(const Blk<double> &b, const AdjBlk &A, int stage, double Bdt, double A_s, cudaStream_t s,
-                      int64_t *launches);
-void adj_launch_moment(const Blk<double> &b, const AdjBlk &A, double t, cudaStream_t s, int64_t *launches);
+// one reversed stage; moment: with the sources' moment gradient at time t
+void adj_launch_stage(const Blk<double> &b, const AdjBlk &A, int stage, double Bdt, double A_s, bool moment, double t,
+                      cudaStream_t s, int64_t *launches);
 void adj_launch_receivers(const Blk<double> &b, const AdjBlk &A, cudaStream_t s, int64_t *launches);
 int upload_tables_adjoint(const void *t);
 

@@ -1919,8 +1919,7 @@ int wql3d_adjoint_step(wql3d_domain *d, int n, double dt) {
   CK(cudaMemcpyAsync(d->cur ? b.F1 : b.F0, A.S[0], bytes, cudaMemcpyDeviceToDevice, d->stream));
   // reversed stages 5..1
   for (int s = 5; s >= 1; --s) {
-    adj_launch_stage(b, A, s, kRkB[s - 1] * dt, kRkA[s - 1], d->stream, &d->launches);
-    adj_launch_moment(b, A, t0 + kRkC[s - 1] * dt, d->stream, &d->launches);
+    adj_launch_stage(b, A, s, kRkB[s - 1] * dt, kRkA[s - 1], true, t0 + kRkC[s - 1] * dt, d->stream, &d->launches);
   }
   CK(cudaGetLastError());
   return WQL3D_OK;
@@ -1964,8 +1963,7 @@ int wql3d_adjoint_step_recorded(wql3d_domain *d, int n, double dt, double t_n, c
     A.E[s] = terms ? dev_in + (5 + s) * ne : nullptr;
   }
   for (int s = 5; s >= 1; --s) {
-    adj_launch_stage(b, A, s, kRkB[s - 1] * dt, kRkA[s - 1], d->stream, &d->launches);
-    adj_launch_moment(b, A, t_n + kRkC[s - 1] * dt, d->stream, &d->launches);
+    adj_launch_stage(b, A, s, kRkB[s - 1] * dt, kRkA[s - 1], true, t_n + kRkC[s - 1] * dt, d->stream, &d->launches);
   }
   CK(cudaGetLastError());
   return WQL3D_OK;
@@ -1992,7 +1990,7 @@ int wql3d_adjoint_rhs(wql3d_domain *d, int bi, const double *R, double *Fbar, do
   CK(cudaMemsetAsync(A.g, 0, sizeof(double) * 3 * V, d->stream));
   if (int rc = put_array<double>(d, d->hb[0], A.DFb, 9, R, 0)) return rc;
   CK(cudaMemcpyAsync(A.S[0], d->cur ? b.F1 : b.F0, sizeof(double) * 9 * V, cudaMemcpyDeviceToDevice, d->stream));
-  adj_launch_stage(b, A, 1, 0.0, 0.0, d->stream, &d->launches);
+  adj_launch_stage(b, A, 1, 0.0, 0.0, false, 0.0, d->stream, &d->launches);
   CK(cudaGetLastError());
   if (int rc = get_array<double>(d, d->hb[0], A.Fb, 9, Fbar, 0)) return rc;
   return get_array<double>(d, d->hb[0], A.g, 3, g, 0);
