@@ -53,6 +53,27 @@ def test_stages_from_a_random_state(wql3d_lib, oracle_lib, mesh, response, pml, 
         assert rel_l2(g.eta(), o.eta()) < 1e-11
 
 
+@pytest.mark.parametrize("n", [(16, 17, 18), (33, 16, 19)])
+@pytest.mark.parametrize("op", [("upwind", 4), ("upwind", 6), ("upwind_drp", 6)])
+@pytest.mark.parametrize("mesh,response", [("cartesian", "anelastic-fQ8"), ("curvilinear", "elastic")])
+def test_upwind_stages_from_a_random_state(wql3d_lib, oracle_lib, mesh, response, op, n):
+    """The upwind pairs at 16 points, twice the widest closure."""
+    p = small_case(mesh=mesh, response=response, n=n)
+    p.fd_type, p.order = op
+    (F, DF), = random_state(p)
+    dt = p.dt()
+    o, g = oracle_lib.OracleDomain(p), _domain(p)
+    for d in (o, g):
+        d.set_fields(F)
+    o.set_rates(DF)
+    g.set_rates_array(DF)
+    for st in (1, 2):
+        o.stage(st, dt)
+        g.stage(st, dt)
+    assert rel_l2(g.rates(), o.rates()) < 1e-12
+    assert rel_l2(g.fields(), o.fields()) < 1e-12
+
+
 @pytest.mark.parametrize("mesh", ["cartesian", "curvilinear"])
 def test_run_after_every_way_of_setting_fields(wql3d_lib, oracle_lib, mesh):
     """Graph-replayed steps, fields set again, the split operations in between,

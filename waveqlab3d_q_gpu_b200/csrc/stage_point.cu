@@ -5,7 +5,7 @@
 
 namespace wql3d {
 
-template <typename T, int MESH, int RESP, bool PML>
+template <typename T, int MESH, int RESP, bool PML, bool UP>
 static void launch_point(Blk<T> &b, const StageCtx &c, const StageArgs &a) {
   // Elastic blocks and FP32 take the flattened points with 6 resident CTAs
   // (the roles' taps are short enough for 80 registers): FP64 ms per step
@@ -17,17 +17,17 @@ static void launch_point(Blk<T> &b, const StageCtx &c, const StageArgs &a) {
   constexpr bool FLAT = sizeof(T) == 4 || RESP == RESP_EL;
   const WarpMap m = warp_map(b);
   const long long n = FLAT ? ((long long)b.nx * b.ny * b.nz + 127) / 128 : (map_warps(b, m) + 3) / 4;
-  k_point<T, MESH, RESP, PML, FLAT, FLAT ? 6 : 4><<<(unsigned)(2 * n), 128, 0, c.stream>>>(b, a, m);
+  k_point<T, MESH, RESP, PML, FLAT, FLAT ? 6 : 4, UP><<<(unsigned)(2 * n), 128, 0, c.stream>>>(b, a, m);
   ++*c.launches;
 }
 
-template <typename T, int MESH, bool PML>
+template <typename T, int MESH, bool PML, bool UP = false>
 static void launch_resp(Blk<T> &b, const StageCtx &c, const StageArgs &a) {
   switch (c.response) {
-    case RESP_EL: launch_point<T, MESH, RESP_EL, PML>(b, c, a); break;
-    case RESP_Q4: launch_point<T, MESH, RESP_Q4, PML>(b, c, a); break;
-    case RESP_Q8: launch_point<T, MESH, RESP_Q8, PML>(b, c, a); break;
-    default: launch_point<T, MESH, RESP_FQ8, PML>(b, c, a); break;
+    case RESP_EL: launch_point<T, MESH, RESP_EL, PML, UP>(b, c, a); break;
+    case RESP_Q4: launch_point<T, MESH, RESP_Q4, PML, UP>(b, c, a); break;
+    case RESP_Q8: launch_point<T, MESH, RESP_Q8, PML, UP>(b, c, a); break;
+    default: launch_point<T, MESH, RESP_FQ8, PML, UP>(b, c, a); break;
   }
 }
 
@@ -37,6 +37,18 @@ void launch_point_stage(Blk<T> &b, int mesh, const StageCtx &c, const StageArgs 
   la.pf = sizeof(T) == 4 ? 1 : 0;   // L2 prefetch of the memory variables (FP32 only: see k_curv_fused)
   bool pml = false;
   for (int f = 0; f < 6; ++f) pml = pml || b.pml_on[f];
+  if (b.fd != 0) {
+    if (mesh == MESH_CART) {
+      launch_resp<T, MESH_CART, false, true>(b, c, la);
+      return;
+    }
+    if (b.foff[6] > 0) {
+      k_curv_face_sat<T><<<(b.foff[6] + 127) / 128, 128, 0, c.stream>>>(b, a.cur);
+      ++*c.launches;
+    }
+    launch_resp<T, MESH_CURV, false, true>(b, c, la);
+    return;
+  }
   if (mesh == MESH_CART) {
     if (pml) launch_resp<T, MESH_CART, true>(b, c, la);
     else launch_resp<T, MESH_CART, false>(b, c, la);
@@ -68,8 +80,12 @@ bool point_stage_ok(const Blk<T> &b, int mesh) {
   const int nax[3] = {b.nx, b.ny, b.nz};
   for (int ax = 0; ax < 3; ++ax)
     if (b.pml_on[2 * ax] && b.pml_on[2 * ax + 1] && 2 * b.npml > nax[ax]) return false;
+  if (b.fd != 0) {
+    for (int f = 0; f < 6; ++f)
+      if (b.pml_on[f]) return false;   // upwind blocks with PML: the generic kernel
+  }
   if (mesh == MESH_CART) return tuning().point && b.sep;
-  return tuning().curv_fused && tuning().lean && !(sizeof(T) == 4 && b.nmech > 0);
+  return tuning().curv_fused && tuning().lean && !(sizeof(T) == 4 && b.nmech > 0 && b.fd == 0);
 }
 
 template <typename T>

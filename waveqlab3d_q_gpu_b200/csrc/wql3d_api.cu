@@ -898,7 +898,7 @@ int setup_block(wql3d_domain *d, int bi) {
                 else omax = std::max(omax, v);
               }
           }
-      b.sep = (omax <= 1e-12 * dmin && b.fd == WQL3D_FD_TRADITIONAL6) ? 1 : 0;
+      b.sep = omax <= 1e-12 * dmin ? 1 : 0;
     }
   }
 
@@ -1016,8 +1016,7 @@ int setup_block(wql3d_domain *d, int bi) {
 template <typename T>
 bool point_path(wql3d_domain *d, int bi) {
   const Blk<T> &b = blk<T>(d, bi);
-  return !tuning().generic && !b.mms && b.fd == WQL3D_FD_TRADITIONAL6 &&
-         point_stage_ok(b, d->hb[bi].mesh);
+  return !tuning().generic && !b.mms && point_stage_ok(b, d->hb[bi].mesh);
 }
 
 // the flux arrays of a curvilinear block on the point path, made current

@@ -148,15 +148,43 @@ __device__ __forceinline__ void axis_any(const Blk<T> &b, int i, const T *__rest
   else axis_closure<T, MESH, ROLE, AX>(b, i, F, V, o, st, d);
 }
 
+// upwind pairs: the forward rows on the velocities, the backward rows on the
+// stresses (or fluxes), from the block's row table (Blk::urowc), four taps'
+// loads at a time (Q8, upwind-4, 61^3 points in FP64: 0.63 ms per step, 1.48
+// through the generic kernel's 255 registers and 8 warps per SM)
+template <typename T, int MESH, int ROLE, int AX>
+__device__ __forceinline__ void axis_upwind(const Blk<T> &b, int i, const T *__restrict__ F, long long V, unsigned o,
+                                            int st, T d[3]) {
+  const int row = up_row(b, ROLE == ROLE_S, i, axis_len<AX>(b));
+  const int cnt = __ldg(b.urown + row);
+  const double *__restrict__ rc = b.urowc + row * 16;
+  const int *__restrict__ ro = b.urowo + row * 16;
+  const T *__restrict__ f0 = tap_array<T, MESH, ROLE, AX, 0>(F, V), *__restrict__ f1 = tap_array<T, MESH, ROLE, AX, 1>(F, V),
+                       *__restrict__ f2 = tap_array<T, MESH, ROLE, AX, 2>(F, V);
+  d[0] = d[1] = d[2] = (T)0;
+#pragma unroll 4
+  for (int k = 0; k < cnt; ++k) {
+    const T c = (T)__ldg(rc + k);
+    const unsigned q = o + (unsigned)(__ldg(ro + k) * st);
+    d[0] = d[0] + c * at(f0, q);
+    d[1] = d[1] + c * at(f1, q);
+    d[2] = d[2] + c * at(f2, q);
+  }
+}
+
 // the nine derivatives of a role at one point, g[a][c] with the axis metric
 // (Cartesian) and 1/h applied.  inner: every lane of the warp has central
-// rows on all three axes
-template <typename T, int MESH, int ROLE>
+// rows on all three axes.  UP: the block's upwind pair
+template <typename T, int MESH, int ROLE, bool UP>
 __device__ __forceinline__ void derivatives(const Blk<T> &b, const T *__restrict__ F, bool inner, int x, int y, int z,
                                             unsigned o, T g[3][3]) {
   const long long V = b.vol;
   const int sy = (int)b.sy, sz = (int)b.sz;
-  if (inner) {
+  if constexpr (UP) {
+    axis_upwind<T, MESH, ROLE, 0>(b, x, F, V, o, 1, g[0]);
+    axis_upwind<T, MESH, ROLE, 1>(b, y, F, V, o, sy, g[1]);
+    axis_upwind<T, MESH, ROLE, 2>(b, z, F, V, o, sz, g[2]);
+  } else if (inner) {
     axis_central<T, MESH, ROLE, 0>(F, V, o, 1, g[0]);
     axis_central<T, MESH, ROLE, 1>(F, V, o, sy, g[1]);
     axis_central<T, MESH, ROLE, 2>(F, V, o, sz, g[2]);
@@ -426,7 +454,7 @@ __device__ __forceinline__ void store_fluxes(const Blk<T> &b, T *__restrict__ G,
 }
 
 // one point of a full stage (flags F_ALL), velocity half
-template <typename T, int MESH, bool PML>
+template <typename T, int MESH, bool PML, bool UP>
 __device__ __forceinline__ void point_v(const Blk<T> &b, const StageArgs &a, bool inner, int x, int y, int z) {
   const long long V = b.vol;
   const unsigned o = (unsigned)pidx(b, x, y, z);
@@ -443,7 +471,7 @@ __device__ __forceinline__ void point_v(const Blk<T> &b, const StageArgs &a, boo
 #pragma unroll
   for (int c = 0; c < 3; ++c) f[c] = at(F + c * V, o);
   T g[3][3];
-  derivatives<T, MESH, ROLE_V>(b, MESH == MESH_CURV ? b.G + (a.cur ? 9 * V : 0) : F, inner, x, y, z, o, g);
+  derivatives<T, MESH, ROLE_V, UP>(b, MESH == MESH_CURV ? b.G + (a.cur ? 9 * V : 0) : F, inner, x, y, z, o, g);
   if (MESH == MESH_CURV && a.rec) {
     T *E = reinterpret_cast<T *>(a.rec);
 #pragma unroll
@@ -461,7 +489,7 @@ __device__ __forceinline__ void point_v(const Blk<T> &b, const StageArgs &a, boo
 }
 
 // one point of a full stage (flags F_ALL), stress half
-template <typename T, int MESH, int RESP, bool PML>
+template <typename T, int MESH, int RESP, bool PML, bool UP>
 __device__ __forceinline__ void point_s(const Blk<T> &b, const StageArgs &a, bool inner, int x, int y, int z) {
   const long long V = b.vol;
   const unsigned o = (unsigned)pidx(b, x, y, z);
@@ -484,7 +512,7 @@ __device__ __forceinline__ void point_s(const Blk<T> &b, const StageArgs &a, boo
   for (int c = 0; c < 6; ++c) df[c] = (b.DF + (3 + c) * V)[o];
   const T lam = at(b.M, o), mu = at(b.M + V, o);
   T g[3][3];
-  derivatives<T, MESH, ROLE_S>(b, F, inner, x, y, z, o, g);
+  derivatives<T, MESH, ROLE_S, UP>(b, F, inner, x, y, z, o, g);
   if constexpr (MESH == MESH_CURV) {
     T u[3][3];
 #pragma unroll
@@ -611,25 +639,25 @@ __device__ __forceinline__ bool flat_index(const Blk<T> &b, int j, int &x, int &
 }
 
 // one role at one point, the warp's lanes agreeing on the straight-line taps
-template <typename T, int MESH, int RESP, bool PML>
+template <typename T, int MESH, int RESP, bool PML, bool UP = false>
 __device__ __forceinline__ void run_role(const Blk<T> &b, const StageArgs &a, int role, int x, int y, int z) {
   const bool c = central_row(b, 0, x, b.nx) && central_row(b, 1, y, b.ny) && central_row(b, 2, z, b.nz);
   const bool inner = __all_sync(__activemask(), c);
-  if (role == ROLE_S) point_s<T, MESH, RESP, PML>(b, a, inner, x, y, z);
-  else point_v<T, MESH, PML>(b, a, inner, x, y, z);
+  if (role == ROLE_S) point_s<T, MESH, RESP, PML, UP>(b, a, inner, x, y, z);
+  else point_v<T, MESH, PML, UP>(b, a, inner, x, y, z);
 }
 
 // CTA pair (2 k, 2 k + 1): the two roles of 128 points.  FLAT: consecutive
 // points of the flattened block (every lane busy; warps straddle row ends),
 // else four warps of the work map m (no warp mixes boundary columns with
 // central ones).
-template <typename T, int MESH, int RESP, bool PML, bool FLAT, int MINB>
+template <typename T, int MESH, int RESP, bool PML, bool FLAT, int MINB, bool UP>
 __global__ void __launch_bounds__(128, MINB) k_point(const __grid_constant__ Blk<T> b,
                                                      const __grid_constant__ StageArgs a, WarpMap m) {
   int x, y, z;
   const int t = (blockIdx.x >> 1) * 128 + threadIdx.x;
   if (FLAT ? !flat_index(b, t, x, y, z) : !warp_point(b, m, t >> 5, t & 31, x, y, z)) return;
-  run_role<T, MESH, RESP, PML>(b, a, blockIdx.x & 1 ? ROLE_S : ROLE_V, x, y, z);
+  run_role<T, MESH, RESP, PML, UP>(b, a, blockIdx.x & 1 ? ROLE_S : ROLE_V, x, y, z);
 }
 
 // The contravariant fluxes of the fields F on planes z0 .. z1 (ghost planes
