@@ -152,8 +152,9 @@ struct wql3d_domain {
   int response = 0;
   int nmech = 0;
   cudaStream_t stream = nullptr;
-  // second stream for the Cartesian near-boundary shell, forked from and
-  // joined back to `stream` every stage (the shell overlaps the interior)
+  // second stream, forked from and joined back to `stream` every stage: the
+  // second block's point kernels, or the near-boundary shell beside the
+  // interior tiles of a full-metric Cartesian block
   cudaStream_t side = nullptr;
   cudaEvent_t fork = nullptr, join = nullptr;
   Alloc mem;
@@ -1030,10 +1031,10 @@ void ensure_fluxes(wql3d_domain *d, int bi) {
 }
 
 template <typename T>
-void launch_stage(wql3d_domain *d, int bi, const StageArgs &a, bool fused = false) {
+void launch_stage(wql3d_domain *d, int bi, const StageArgs &a, bool fused = false, cudaStream_t stream = nullptr) {
   Blk<T> &b = blk<T>(d, bi);
   const int mesh = d->hb[bi].mesh;
-  StageCtx c{d->stream, d->response, &d->launches, d->side, d->fork, d->join};
+  StageCtx c{stream ? stream : d->stream, d->response, &d->launches, d->side, d->fork, d->join};
   const bool special = tuning().generic || b.mms || b.fd != WQL3D_FD_TRADITIONAL6;
   if (a.flags == F_ALL && point_path<T>(d, bi)) {
     ensure_fluxes<T>(d, bi);
@@ -1066,7 +1067,20 @@ int enqueue_stage(wql3d_domain *d, int stage, double dt, int flags, void *rec = 
     launch_iface<T>(d->iface, blk<T>(d, 0), blk<T>(d, 1), a, d->stream);
     d->launches++;
   }
-  for (int i = 0; i < d->nblocks; ++i) launch_stage<T>(d, i, a, true);
+  if (d->nblocks == 2 && flags == F_ALL && point_path<T>(d, 0) && point_path<T>(d, 1)) {
+    // the blocks share no point after the interface terms: the second on the
+    // side stream, so that the one's last wave of CTAs runs beside the other's
+    // (two-block rupture of 2 x 51 x 81 x 61 points, FP64: 0.592 -> 0.554 ms per step)
+    for (int i = 0; i < 2; ++i) ensure_fluxes<T>(d, i);
+    CK(cudaEventRecord(d->fork, d->stream));
+    CK(cudaStreamWaitEvent(d->side, d->fork, 0));
+    launch_stage<T>(d, 1, a, true, d->side);
+    CK(cudaEventRecord(d->join, d->side));
+    launch_stage<T>(d, 0, a, true);
+    CK(cudaStreamWaitEvent(d->stream, d->join, 0));
+  } else {
+    for (int i = 0; i < d->nblocks; ++i) launch_stage<T>(d, i, a, true);
+  }
   if (flags & F_UPDATE) d->cur ^= 1;
   return WQL3D_OK;
 }
