@@ -10,14 +10,18 @@ static void launch_point(Blk<T> &b, const StageCtx &c, const StageArgs &a) {
   // Elastic blocks and FP32 take the flattened points with 6 resident CTAs
   // (the roles' taps are short enough for 80 registers): FP64 ms per step
   // 0.56 flattened / 0.68 by the warp map on 83 x 121 x 67 curvilinear points,
-  // 0.69 / 0.71 on Cartesian 101^3.  Memory variables in FP64 want the
-  // registers of 4 CTAs and no boundary columns among a warp's central ones:
-  // 22.8 by the map / 23.4 flattened on the two-block Q8 hill of 201^3 points
-  // (27.7 with 6 CTAs), 1.57 / 1.77 on Q4 with PML of 93 x 118 x 75.
+  // 0.69 / 0.71 on Cartesian 101^3 (8 CTAs flattened: 0.61 and 0.76).  FP32 with at
+  // most 4 mechanisms has room for 8 CTAs: 0.546 against 0.603 on Cartesian
+  // 101^3, 1.21 against 1.24 on Q4 with PML of 93 x 118 x 75 (fQ8: 7.06 against
+  // 6.29 on 96 x 160 x 128 twice, so 6 there).  Memory variables in FP64 want
+  // the registers of 4 CTAs and no boundary columns among a warp's central
+  // ones: 22.8 by the map / 23.4 flattened on the two-block Q8 hill of 201^3
+  // points (27.7 with 6 CTAs), 1.57 / 1.77 on Q4 with PML of 93 x 118 x 75.
   constexpr bool FLAT = sizeof(T) == 4 || RESP == RESP_EL;
   const WarpMap m = warp_map(b);
   const long long n = FLAT ? ((long long)b.nx * b.ny * b.nz + 127) / 128 : (map_warps(b, m) + 3) / 4;
-  k_point<T, MESH, RESP, PML, FLAT, FLAT ? 6 : 4, UP><<<(unsigned)(2 * n), 128, 0, c.stream>>>(b, a, m);
+  constexpr int MINB = !FLAT ? 4 : sizeof(T) == 4 && (RESP == RESP_EL || RESP == RESP_Q4) ? 8 : 6;
+  k_point<T, MESH, RESP, PML, FLAT, MINB, UP><<<(unsigned)(2 * n), 128, 0, c.stream>>>(b, a, m);
   ++*c.launches;
 }
 

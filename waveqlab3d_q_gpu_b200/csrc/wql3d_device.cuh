@@ -74,7 +74,8 @@ struct Blk {
   T *F0, *F1;           // field buffers (9 components each)
   T *DF;                // rates (9 components)
   T *FC;                // FP32 path: Kahan compensation for F (9 components)
-  T *G;                 // curvilinear: 18 derivative terms per point from k_curv_grad (see there)
+  T *G;                 // curvilinear: the stress fluxes of either field buffer (9 each, wql3d_point.cuh), or the
+                        // three-pass split's 18 derivative terms (see k_curv_grad)
   T *S6;                // curvilinear anelastic: per stress component the sum of the memory variables
   const double *X;      // physical coordinates x, y, z (FP64, field layout)
   int mms;              // manufactured-solution forcing and boundary data
@@ -149,8 +150,8 @@ struct StageArgs {
   int stage;            // 1..5
   double A, Bdt, dt;
   const DevTime *time;
-  int pf = 0;           // k_curv_fused: 1 = L2 prefetch of the memory variables on entry
-  // k_curv_fused: when set, every point writes the derivative terms of the
+  int pf = 0;           // 1 = L2 prefetch of the memory variables on entry (k_curv_fused, point kernels)
+  // curvilinear stage kernels: when set, every point writes the derivative terms of the
   // stage input the adjoint's material gradient needs (9 components, field
   // layout): e = (U0, U4, U8, U3 + U1, U6 + U2, U7 + U5) and the stress-flux
   // sums (S0 + S3 + S6, S1 + S4 + S7, S2 + S5 + S8)

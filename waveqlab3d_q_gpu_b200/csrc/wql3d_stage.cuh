@@ -1,5 +1,5 @@
 // Host-side launchers of the per-block stage kernels, one family per
-// translation unit (stage_cart.cu, stage_curv.cu, stage_generic.cu), each
+// translation unit (stage_point.cu, stage_cart.cu, stage_curv.cu, stage_generic.cu), each
 // compiled once per precision (WQL3D_REAL = double / float) so that the
 // heavy kernel templates build in parallel.  wql3d_api.cu calls them through
 // the declarations below.
@@ -29,8 +29,9 @@ struct StageCtx {
   cudaStream_t stream;
   int response;       // RESP_*
   int64_t *launches;  // kernel-launch counter of the owning domain
-  // optional second stream and fork / join events: the Cartesian shell runs
-  // there, concurrently with the interior (disjoint points, read-only F)
+  // optional second stream and fork / join events: the shell of a tile-kernel
+  // Cartesian block runs there, concurrently with the interior (disjoint
+  // points, read-only F)
   cudaStream_t side = nullptr;
   cudaEvent_t fork = nullptr, join = nullptr;
 };
@@ -81,7 +82,8 @@ inline int upload_tables_here(const ConstTables &t) {
   return (int)e;
 }
 
-// Cartesian fused stage (flags == F_ALL): strict interior + near-boundary shell
+// Cartesian fused stage (flags == F_ALL) of the blocks the point kernels do not
+// take: strict interior + near-boundary shell
 template <typename T>
 void launch_cart_stage(Blk<T> &b, const StageCtx &c, const StageArgs &a);
 // curvilinear split stage: derivative pass, memory variables, face SATs, point update
@@ -96,8 +98,9 @@ template <typename T>
 void launch_fluxes(const Blk<T> &b, const StageCtx &c, int cur, int z0, int z1);
 template <typename T>
 bool point_stage_ok(const Blk<T> &b, int mesh);
-// true when the block's full curvilinear stages run k_curv_fused (which can
-// record the adjoint's derivative terms, StageArgs::rec)
+// true when the block's full curvilinear stages are one pass (k_curv_fused or
+// the point kernels, which can record the adjoint's derivative terms,
+// StageArgs::rec)
 template <typename T>
 bool curv_stage_fused(const Blk<T> &b);
 // generic per-point kernel (any flags, MMS, both meshes)
