@@ -32,16 +32,8 @@ struct RoleComps {
 };
 
 template <int AX, typename T>
-__device__ __forceinline__ long long axis_stride(const Blk<T> &b) {
-  return AX == 0 ? 1 : AX == 1 ? b.sy : b.sz;
-}
-template <int AX, typename T>
 __device__ __forceinline__ int axis_len(const Blk<T> &b) {
   return AX == 0 ? b.nx : AX == 1 ? b.ny : b.nz;
-}
-template <int AX, typename T>
-__device__ __forceinline__ T axis_ih(const Blk<T> &b) {
-  return AX == 0 ? b.ihq : AX == 1 ? b.ihr : b.ihs;
 }
 template <int AX, typename T>
 __device__ __forceinline__ T axis_metric(const Blk<T> &b, int i) {
