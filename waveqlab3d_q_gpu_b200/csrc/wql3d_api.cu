@@ -683,9 +683,9 @@ int setup_block(wql3d_domain *d, int bi) {
   int iz = bd.pml[4] ? std::max(np, w) : w, fz = bd.pml[5] ? std::max(np, w) : w;
   if (b.open_lo[2]) iz = 0;   // open faces: the central row reaches the face
   if (b.open_hi[2]) fz = 0;
-  b.lo[0] = ix + 1; b.hi[0] = h.nq - fx;
-  b.lo[1] = iy + 1; b.hi[1] = h.nr - fy;
-  b.lo[2] = iz + 1; b.hi[2] = h.ns - fz;
+  interior_range(h.nq, ix, fx, b.lo[0], b.hi[0]);
+  interior_range(h.nr, iy, fy, b.lo[1], b.hi[1]);
+  interior_range(h.ns, iz, fz, b.lo[2], b.hi[2]);
 
   Alloc &M = d->mem;
   CK(M.get(&b.F0, 9 * vol));

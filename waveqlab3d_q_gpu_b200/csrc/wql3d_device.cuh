@@ -2074,6 +2074,16 @@ __global__ void __launch_bounds__(128, MINB) k_curv_fused(Blk<T> b, StageArgs a)
   }
 }
 
+// Strict-interior rows lo .. hi of an axis of n points that keeps `left` and
+// `right` rows out of it.  Where those meet or cross (the two PML slabs of an
+// axis overlap, or a slab reaches the other closure) the range is empty with
+// hi = lo - 1: bounds that crossed would make the shell's parts below overlap,
+// so that two threads update a point, and leave others out.
+inline void interior_range(int n, int left, int right, int &lo, int &hi) {
+  lo = (left < n ? left : n) + 1;
+  hi = n - right > lo - 1 ? n - right : lo - 1;
+}
+
 // Number of near-boundary (shell) points: everything outside the strict
 // interior box, split into z-slabs, y-slabs of the middle planes and x-slabs
 // of the middle rows.
@@ -2087,7 +2097,7 @@ __host__ __device__ inline long long shell_count(const Blk<T> &b) {
 }
 
 template <typename T>
-__device__ inline void shell_decode(const Blk<T> &b, int idx, int &x, int &y, int &z) {
+__host__ __device__ inline void shell_decode(const Blk<T> &b, int idx, int &x, int &y, int &z) {
   const int nx = b.nx, nxy = b.nx * b.ny;
   const int n_zlo = nxy * (b.lo[2] - 1), n_zhi = nxy * (b.nz - b.hi[2]);
   if (idx < n_zlo) {
