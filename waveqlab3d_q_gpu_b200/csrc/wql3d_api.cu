@@ -1067,7 +1067,7 @@ int enqueue_stage(wql3d_domain *d, int stage, double dt, int flags, void *rec = 
     launch_iface<T>(d->iface, blk<T>(d, 0), blk<T>(d, 1), a, d->stream);
     d->launches++;
   }
-  if (d->nblocks == 2 && flags == F_ALL && point_path<T>(d, 0) && point_path<T>(d, 1)) {
+  if (tuning().overlap && d->nblocks == 2 && flags == F_ALL && point_path<T>(d, 0) && point_path<T>(d, 1)) {
     // the blocks share no point after the interface terms: the second on the
     // side stream, so that the one's last wave of CTAs runs beside the other's
     // (two-block rupture of 2 x 51 x 81 x 61 points, FP64: 0.592 -> 0.554 ms per step)

@@ -44,7 +44,8 @@ struct Tuning {
   int curv_fused = 1; // curvilinear stage in one pass, k_curv_fused (0: derivative / memory-variable / point passes)
   int fused_minb = 0; // k_curv_fused resident 128-thread blocks per SM: 3 (default), 2 or 4 in FP64; 4 (default), 5 or 6 in FP32
   int mvpf = -1;      // k_curv_fused: L2 prefetch of the memory variables on entry (-1: FP32 only)
-  int overlap = 1;    // Cartesian stage: shell on the side stream, concurrent with the interior
+  int overlap = 1;    // side stream in use: the shell beside the interior tiles, the second block's point kernels beside
+                      // the first's (0: every stage on one stream)
   int point = 1;      // separable Cartesian stages through the point kernels (0 when WQL3D_TMA is set: the tile kernel)
   int tma = 0;        // Cartesian interior: 1 = planes filled by TMA box loads (default: cp.async, measured faster);
                       // 2 = TMA waits with no copies issued (test of the bounded waits and the stall status)
