@@ -1,0 +1,40 @@
+"""Batched shots on each of the batch's launch routes: the point kernels, and
+interior tiles beside a near-boundary shell (separable FP32 elastic shots above
+2^20 points, where they are most of the batch; shots with a full metric, which the single-precision closure
+literal gives a Cartesian block).  The launches per step say which route ran:
+one sample and one advance launch, then per stage one launch of every class on
+the point kernels and two of every class on the tiles."""
+import pytest
+
+from cases import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+NSTEPS = 12
+
+
+def _single(p, precision="fp64"):
+    from waveqlab3d_q_gpu_b200.domain import Domain
+    g = Domain(p, precision=precision, nsteps_hint=NSTEPS)
+    g.run(NSTEPS)
+    F, s = g.fields(0), g.seismograms(0)
+    g.close()
+    return F, s
+
+
+def test_fp32_elastic_tiles_above_2_20_points(wql3d_lib):
+    """101^3 points (below the line) and 102^3 (above, and the larger part) in one batch.  FP32 with
+    compensated state stays within a few rounding errors (6e-8 each, of every
+    stage's derivatives) of FP64 over 12 steps: 1e-5 as in the other
+    FP32-batch test, far below what a missed point or tap would leave."""
+    from waveqlab3d_q_gpu_b200.shots import ShotBatch, random_shot
+    ps = [random_shot(40 + n, n, n, steps=NSTEPS + 2, response="elastic") for n in (101, 102)]
+    b = ShotBatch(ps, precision="fp32", nsteps_hint=NSTEPS)
+    b.run(NSTEPS)
+    b.synchronize()
+    assert b.kernel_launches() == NSTEPS * (2 + 5 * (1 + 2))
+    for p, d in zip(ps, b.domains):
+        F, _ = _single(p)   # no wave has reached the stations yet: fields only
+        assert rel_l2(d.fields(0)[:3], F[:3]) < 1e-5
+        assert rel_l2(d.fields(0)[3:], F[3:]) < 1e-5
+    b.close()

@@ -5,8 +5,8 @@
 // descriptor in shared memory before running the same tile / point bodies as
 // the per-domain kernels (interior_split_tile, point_update, sample_block).
 //
-// Work lists: every CTA belongs to one shot.  Separable blocks run the two
-// roles of the point kernels (k_batch_point, pairs of CTAs over 128
+// Work lists: every CTA belongs to one shot.  Most separable blocks run the
+// two roles of the point kernels (k_batch_point, pairs of CTAs over 128
 // consecutive points); the others an interior launch over their 32 x 4 x
 // zchunk tiles and a shell launch over their near-boundary points in chunks of
 // 128 (each shot's chunk count rounded up, so no CTA straddles two shots).  A
@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(128, MINB) k_batch_point(BatchClass<T> C, cons
   run_role<T, MESH_CART, RESP, false>(sb, la, s_local & 1 ? ROLE_S : ROLE_V, x, y, z);
 }
 
-template <typename T, int RESP>
+template <typename T, int RESP, bool SEP>
 __global__ void __launch_bounds__(128, 3) k_batch_shell(BatchClass<T> C, StageArgs a) {
   __shared__ __align__(16) Blk<T> sb;
   __shared__ int s_shot, s_local;
@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(128, 3) k_batch_shell(BatchClass<T> C, StageAr
   shell_decode(sb, (int)idx, x, y, z);
   StageArgs la = a;
   la.time = C.times[s_shot];
-  point_update<T, MESH_CART, RESP, false, false, true>(sb, la, x, y, z);
+  point_update<T, MESH_CART, RESP, SEP, false, true>(sb, la, x, y, z);
 }
 
 // stage-1 station samples of every shot: one CTA per shot
@@ -126,7 +126,7 @@ __global__ void k_batch_advance(DevTime *const *times, int n, double dt) {
 template <typename T, int RESP>
 void launch_class(const BatchClass<T> &C, const StageArgs &a, int zchunk, int minb, cudaStream_t s, int part,
                   int64_t *launches) {
-  if (C.sep) {
+  if (C.point) {
     if (part != 0 || C.tiles <= 0) return;
     StageArgs la = a;
     la.pf = sizeof(T) == 4 ? 1 : 0;
@@ -148,7 +148,10 @@ void launch_class(const BatchClass<T> &C, const StageArgs &a, int zchunk, int mi
     ++*launches;
   }
   if (part == 1 && C.shell_ctas > 0) {
-    k_batch_shell<T, RESP><<<C.shell_ctas, 128, 0, s>>>(C, a);
+    // separable blocks come here in FP32 elastic classes only (batch_tiles_faster)
+    if (sizeof(T) == 4 && RESP == RESP_EL && C.sep)
+      k_batch_shell<T, RESP, sizeof(T) == 4 && RESP == RESP_EL><<<C.shell_ctas, 128, 0, s>>>(C, a);
+    else k_batch_shell<T, RESP, false><<<C.shell_ctas, 128, 0, s>>>(C, a);
     ++*launches;
   }
 }
@@ -169,6 +172,17 @@ void launch_part(const BatchClass<T> *classes, int ncls, const StageArgs &a, int
 }
 
 }  // namespace
+
+// Shots whose tile kernel is faster than the point kernels where they make up
+// the batch: FP32 elastic above 2^20 points.  ms per step, tiles beside the
+// shell / point kernels: 8 shots of 80^3 2.96 / 2.67, of 96^3 4.62 / 4.64, 6 of
+// 104^3 4.11 / 4.41, 4 of 128^3 4.75 / 5.26, 3 of 160^3 6.41 / 7.60.  FP64
+// elastic and Q4 in either precision gain from the point kernels at every size
+// from 48^3 to 192^3 (1.08 to 1.85 times as fast).
+template <typename T>
+bool batch_tiles_faster(const Blk<T> &b) {
+  return sizeof(T) == 4 && b.nmech == 0 && (long long)b.nx * b.ny * b.nz > 1 << 20;
+}
 
 template <typename T>
 void launch_batch_stage(const BatchClass<T> *classes, int ncls, const StageArgs &a, int zchunk, int minb,
@@ -201,6 +215,7 @@ void launch_batch_advance(DevTime *const *times, int nshots, double dt, cudaStre
   ++*launches;
 }
 
+template bool batch_tiles_faster<WQL3D_REAL>(const Blk<WQL3D_REAL> &);
 template void launch_batch_stage<WQL3D_REAL>(const BatchClass<WQL3D_REAL> *, int, const StageArgs &, int,
                                              int, cudaStream_t, cudaStream_t, cudaEvent_t, cudaEvent_t, int64_t *);
 template void launch_batch_sample<WQL3D_REAL>(const Blk<WQL3D_REAL> *, DevTime *const *, int, int, int,

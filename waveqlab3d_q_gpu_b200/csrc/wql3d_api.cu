@@ -2144,13 +2144,13 @@ struct wql3d_batch {
   void *blks = nullptr;           // device array of Blk<T>
   DevTime **times = nullptr;      // device array of the shots' DevTime pointers
   struct Cls {
-    int resp = 0, sep = 0;
+    int resp = 0, sep = 0, point = 0;
     std::vector<int> shots;
     int *d_shots = nullptr, *d_tile = nullptr, *d_shell = nullptr;
     int tiles = 0, shell_ctas = 0;
-  } cls[8];
+  } cls[12];
   int zchunk = 12;
-  int minb = 6;                   // resident CTAs of the point kernels
+  int minb = 6;                   // resident CTAs of the point kernels (FP32: 8 to begin with)
   bool points = false;            // every class runs the point kernels: minb is tuned, else zchunk
   int tuned = 0;
   int cur = 0;
@@ -2173,7 +2173,7 @@ int batch_tiles(wql3d_batch *bt) {
       const int *lo = bt->fp32 ? d->bf[0].lo : d->bd[0].lo, *hi = bt->fp32 ? d->bf[0].hi : d->bd[0].hi;
       const int nxi = hi[0] - lo[0] + 1, nyi = hi[1] - lo[1] + 1, nzi = hi[2] - lo[2] + 1;
       const long long np = (long long)d->hb[0].nq * d->hb[0].nr * d->hb[0].ns;
-      const int t = c.sep ? 2 * (int)((np + 127) / 128) : (nxi > 0 && nyi > 0 && nzi > 0)
+      const int t = c.point ? 2 * (int)((np + 127) / 128) : (nxi > 0 && nyi > 0 && nzi > 0)
                         ? ((nxi + 31) / 32) * ((nyi + 3) / 4) * ((nzi + bt->zchunk - 1) / bt->zchunk) : 0;
       pre[i + 1] = pre[i] + t;
     }
@@ -2187,13 +2187,14 @@ int batch_tiles(wql3d_batch *bt) {
 template <typename T>
 void batch_enqueue_step(wql3d_batch *bt, double dt, int w_stride) {
   launch_batch_sample<T>((const Blk<T> *)bt->blks, bt->times, bt->n, bt->cur, w_stride, bt->stream, &bt->launches);
-  BatchClass<T> cl[8];
+  BatchClass<T> cl[12];
   int ncl = 0;
   for (auto &c : bt->cls) {
     if (c.shots.empty()) continue;
     BatchClass<T> &b = cl[ncl++];
     b.resp = c.resp;
     b.sep = c.sep;
+    b.point = c.point;
     b.nshots = (int)c.shots.size();
     b.shots = c.d_shots;
     b.tile_prefix = c.d_tile;
@@ -2349,16 +2350,33 @@ int wql3d_batch_create(wql3d_domain *const *domains, int32_t n, wql3d_batch **ou
   if (cudaMemcpyAsync(bt->blks, hb.data(), hb.size(), cudaMemcpyHostToDevice, bt->stream) != cudaSuccess ||
       cudaMemcpyAsync(bt->times, ht.data(), sizeof(DevTime *) * n, cudaMemcpyHostToDevice, bt->stream) != cudaSuccess)
     return bad(fail(WQL3D_ECUDA, "batch descriptor upload"));
-  // classes: response x separable shell
+  // Separable shots run the point kernels; those with faster tiles take the
+  // tiles where they are more than half of the batch or 2^23 points.  With fewer
+  // the launches of their own cost what the tiles save: eight FP32 shots with one
+  // of 128^3 elastic 6.72 ms per step against 6.67, 48 shots of 64^3 to 192^3
+  // with 36 of 111 million points in such shots 99.5 against 103.3.
+  long long points = 0, large = 0;
+  for (int i = 0; i < n; ++i) {
+    const wql3d_domain *d = domains[i];
+    const long long np = (long long)d->hb[0].nq * d->hb[0].nr * d->hb[0].ns;
+    points += np;
+    if (fp32 ? d->bf[0].sep && batch_tiles_faster(d->bf[0]) : d->bd[0].sep && batch_tiles_faster(d->bd[0])) large += np;
+  }
+  const bool tiles = 2 * large > points || large > 1 << 23;
+  // classes: response x (full metric, separable tiles, point kernels)
   for (int i = 0; i < n; ++i) {
     const int sep = fp32 ? domains[i]->bf[0].sep : domains[i]->bd[0].sep;
-    auto &c = bt->cls[domains[i]->response * 2 + (sep ? 1 : 0)];
+    const bool faster = fp32 ? batch_tiles_faster(domains[i]->bf[0]) : batch_tiles_faster(domains[i]->bd[0]);
+    const int point = sep && !(tiles && faster) ? 1 : 0;
+    auto &c = bt->cls[domains[i]->response * 3 + (point ? 2 : sep ? 1 : 0)];
     c.resp = domains[i]->response;
     c.sep = sep ? 1 : 0;
+    c.point = point;
     c.shots.push_back(i);
   }
+  bt->minb = fp32 ? 8 : 6;
   bt->points = true;
-  for (const auto &c : bt->cls) bt->points = bt->points && (c.shots.empty() || c.sep);
+  for (const auto &c : bt->cls) bt->points = bt->points && (c.shots.empty() || c.point);
   for (auto &c : bt->cls) {
     if (c.shots.empty()) continue;
     const size_t m = c.shots.size();

@@ -11,16 +11,18 @@ namespace wql3d {
 // variant (separable or full-metric shell)
 template <typename T>
 struct BatchClass {
-  int resp, sep;
+  int resp, sep, point;    // sep: separable metric; point: the shots run the point kernels
   int nshots;              // shots of this class
   const int *shots;        // their indices in the batch
-  const int *tile_prefix;  // CTAs of the point kernel (sep) or interior tiles: nshots + 1 offsets
-  const int *shell_prefix; // shell CTAs (128 points each; full-metric blocks): nshots + 1 offsets
+  const int *tile_prefix;  // CTAs of the point kernel or interior tiles: nshots + 1 offsets
+  const int *shell_prefix; // shell CTAs (128 points each; beside interior tiles): nshots + 1 offsets
   int tiles, shell_ctas;   // totals
   const Blk<T> *blks;      // every shot's block descriptor (device)
   DevTime *const *times;   // every shot's step time / sample counter (device)
 };
 
+template <typename T>
+bool batch_tiles_faster(const Blk<T> &b);
 // zchunk: planes of an interior tile; minb: resident CTAs the point kernels
 // are compiled for (3 to 8).  side != nullptr: the shells run on the side stream (fork / join events),
 // concurrently with the interior tiles
