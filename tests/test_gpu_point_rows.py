@@ -1,0 +1,52 @@
+"""Elastic Cartesian blocks on both sides of the launch rules that depend on
+their size: rows of 96 (with PML) and 125 points and more are mapped to warps
+row by row, shorter ones as flattened points; FP64 blocks without PML whose
+shortest axis has 139 points run the interior tiles beside the shell (two
+launches a stage instead of one).
+
+Tolerances are those of the single-stage parity tests: 1e-12 relative on rates
+and fields after two stages from a random state; FP32 against FP64 on the same
+state 2e-5, velocities and stresses apart."""
+import pytest
+
+from cases import random_state, rel_l2, small_case
+
+pytestmark = pytest.mark.gpu
+
+
+def _stages(oracle, p, precisions):
+    from waveqlab3d_q_gpu_b200.domain import Domain
+    (F, DF), = random_state(p)
+    o = oracle.OracleDomain(p)
+    ds = [Domain(p, precision=q) for q in precisions]
+    launches = ds[0].kernel_launches()
+    for d in [o] + ds:
+        d.set_fields(F)
+    o.set_rates(DF)
+    for d in ds:
+        d.set_rates_array(DF)
+    for st in (1, 2):
+        for d in [o] + ds:
+            d.stage(st, p.dt())
+    launches = (ds[0].kernel_launches() - launches) / 2
+    Fo = o.fields()
+    assert rel_l2(ds[0].rates(), o.rates()) < 1e-12
+    assert rel_l2(ds[0].fields(), Fo) < 1e-12
+    for d in ds[1:]:
+        assert rel_l2(d.fields()[:3], Fo[:3]) < 2e-5
+        assert rel_l2(d.fields()[3:], Fo[3:]) < 2e-5
+    for d in ds:
+        d.close()
+    return launches
+
+
+@pytest.mark.parametrize("nx,pml", [(95, True), (96, True), (97, True), (128, True), (124, False), (125, False),
+                                    (126, False), (140, False)])
+def test_row_lengths(wql3d_lib, oracle_lib, nx, pml):
+    p = small_case(response="elastic", pml=pml, n=(nx, 15, 16))
+    assert _stages(oracle_lib, p, ("fp64", "fp32")) == 1
+
+
+@pytest.mark.parametrize("n,launches", [((139, 139, 139), 2), ((139, 138, 140), 1)])
+def test_tiles_from_139_points_an_axis(wql3d_lib, oracle_lib, n, launches):
+    assert _stages(oracle_lib, small_case(response="elastic", n=n), ("fp64",)) == launches

@@ -5,24 +5,43 @@
 
 namespace wql3d {
 
-template <typename T, int MESH, int RESP, bool PML, bool UP>
-static void launch_point(Blk<T> &b, const StageCtx &c, const StageArgs &a) {
-  // Elastic blocks and FP32 take the flattened points with 6 resident CTAs
-  // (the roles' taps are short enough for 80 registers): FP64 ms per step
-  // 0.56 flattened / 0.68 by the warp map on 83 x 121 x 67 curvilinear points,
-  // 0.69 / 0.71 on Cartesian 101^3 (8 CTAs flattened: 0.61 and 0.76).  FP32 with at
-  // most 4 mechanisms has room for 8 CTAs: 0.546 against 0.603 on Cartesian
-  // 101^3, 1.21 against 1.24 on Q4 with PML of 93 x 118 x 75 (fQ8: 7.06 against
-  // 6.29 on 96 x 160 x 128 twice, so 6 there).  Memory variables in FP64 want
-  // the registers of 4 CTAs and no boundary columns among a warp's central
-  // ones: 22.8 by the map / 23.4 flattened on the two-block Q8 hill of 201^3
-  // points (27.7 with 6 CTAs), 1.57 / 1.77 on Q4 with PML of 93 x 118 x 75.
-  constexpr bool FLAT = sizeof(T) == 4 || RESP == RESP_EL;
+template <typename T, int MESH, int RESP, bool PML, bool UP, bool FLAT, int MINB>
+static void launch_as(Blk<T> &b, const StageCtx &c, const StageArgs &a) {
   const WarpMap m = warp_map(b);
   const long long n = FLAT ? ((long long)b.nx * b.ny * b.nz + 127) / 128 : (map_warps(b, m) + 3) / 4;
-  constexpr int MINB = !FLAT ? 4 : sizeof(T) == 4 && (RESP == RESP_EL || RESP == RESP_Q4) ? 8 : 6;
   k_point<T, MESH, RESP, PML, FLAT, MINB, UP><<<(unsigned)(2 * n), 128, 0, c.stream>>>(b, a, m);
   ++*c.launches;
+}
+
+template <typename T, int MESH, int RESP, bool PML, bool UP>
+static void launch_point(Blk<T> &b, const StageCtx &c, const StageArgs &a) {
+  if constexpr (RESP == RESP_EL && MESH == MESH_CART && !UP) {
+    // Elastic Cartesian blocks: the flattened points while rows are short, the
+    // warp map (its warps start on their rows' lines) from 125 points a row, 96
+    // with PML.  FP64 with 5 and 6 resident CTAs, FP32 with 8; ms per step,
+    // flattened / mapped:
+    //              81^3         101^3        137^3        160^3        200 x 90 x 200  90 x 200 x 200
+    //   FP64       0.39 / 0.47  0.69 / 0.73  1.72 / 1.53  2.50 / 2.34  2.46 / 1.96     2.27 / 2.48
+    //   FP64, PML  0.77 / 0.77  1.48 / 1.39               4.99 / 3.49
+    //   FP32       0.31 / 0.36  0.56 / 0.58  1.41 / 1.29  2.12 / 1.94  1.89 / 1.66     2.00 / 2.10
+    //   FP32, PML  0.55 / 0.57  1.04 / 1.00               3.63 / 2.69
+    // FP64 flattened with 6 CTAs spills 136 bytes (272 with PML; 5 CTAs: none, 32):
+    // 0.70 at 101^3, 0.088 against 0.082 at 41^3.
+    if (b.nx >= (PML ? 96 : 125)) launch_as<T, MESH, RESP, PML, UP, false, sizeof(T) == 4 ? 8 : 6>(b, c, a);
+    else launch_as<T, MESH, RESP, PML, UP, true, sizeof(T) == 4 ? 8 : 5>(b, c, a);
+  } else {
+    // The other elastic blocks and FP32 take the flattened points with 6 resident
+    // CTAs (FP64 ms per step 0.56 flattened / 0.68 by the warp map on
+    // 83 x 121 x 67 curvilinear points).  FP32 with at most 4 mechanisms has room
+    // for 8 CTAs: 1.21 against 1.24 on Q4 with PML of 93 x 118 x 75 (fQ8: 7.06
+    // against 6.29 on 96 x 160 x 128 twice, so 6 there).  Memory variables in FP64
+    // want the registers of 4 CTAs and no boundary columns among a warp's central
+    // ones: 22.8 by the map / 23.4 flattened on the two-block Q8 hill of 201^3
+    // points (27.7 with 6 CTAs), 1.57 / 1.77 on Q4 with PML of 93 x 118 x 75.
+    constexpr bool FLAT = sizeof(T) == 4 || RESP == RESP_EL;
+    constexpr int MINB = !FLAT ? 4 : sizeof(T) == 4 && (RESP == RESP_EL || RESP == RESP_Q4) ? 8 : 6;
+    launch_as<T, MESH, RESP, PML, UP, FLAT, MINB>(b, c, a);
+  }
 }
 
 template <typename T, int MESH, bool PML, bool UP = false>
@@ -73,6 +92,19 @@ void launch_point_stage(Blk<T> &b, int mesh, const StageCtx &c, const StageArgs 
   }
 }
 
+// FP64 elastic Cartesian blocks without PML whose shortest axis has 139 points
+// or more: the tile kernel beside the shell is the faster one there (ms per
+// step, tiles / point kernel: 137^3 1.55 / 1.53, 145 x 141 x 139 1.75 / 1.82, 160^3 2.29 /
+// 2.34, 201^3 4.14 / 4.22; a short axis makes the shell large: 200 x 200 x 90
+// 1.97 / 1.86, 160 x 160 x 31 0.66 / 0.50).
+template <typename T>
+static bool tiles_faster(const Blk<T> &b) {
+  if (sizeof(T) == 4 || b.nmech > 0 || b.nx < 139 || b.ny < 139 || b.nz < 139) return false;
+  for (int f = 0; f < 6; ++f)
+    if (b.pml_on[f]) return false;
+  return true;
+}
+
 // The point kernels keep one PML slab per axis: blocks whose two slabs on an
 // axis overlap (2 npml > n) take the generic passes.  Cartesian blocks need a
 // separable metric.  FP32 curvilinear blocks with memory variables stay with
@@ -88,7 +120,7 @@ bool point_stage_ok(const Blk<T> &b, int mesh) {
     for (int f = 0; f < 6; ++f)
       if (b.pml_on[f]) return false;   // upwind blocks with PML: the generic kernel
   }
-  if (mesh == MESH_CART) return tuning().point && b.sep;
+  if (mesh == MESH_CART) return tuning().point && b.sep && (b.fd != 0 || !tiles_faster(b));
   return tuning().curv_fused && tuning().lean && !(sizeof(T) == 4 && b.nmech > 0 && b.fd == 0);
 }
 
