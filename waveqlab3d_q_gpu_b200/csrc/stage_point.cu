@@ -29,7 +29,18 @@ static void launch_point(Blk<T> &b, const StageCtx &c, const StageArgs &a) {
     // 0.70 at 101^3, 0.088 against 0.082 at 41^3.
     if (b.nx >= (PML ? 96 : 125)) launch_as<T, MESH, RESP, PML, UP, false, sizeof(T) == 4 ? 8 : 6>(b, c, a);
     else launch_as<T, MESH, RESP, PML, UP, true, sizeof(T) == 4 ? 8 : 5>(b, c, a);
-  } else {
+  } else if constexpr (RESP == RESP_EL && MESH == MESH_CURV && PML) {
+    // Elastic curvilinear blocks with PML: the same line at 96 points a row, FP64
+    // with 5 resident CTAs (6 spill 32 to 40 bytes), FP32 with 8; ms per step,
+    // k_curv_fused / flattened / mapped (FP64 flattened with 6 CTAs):
+    //          61^3                       101^3                      160^3                      160 x 31 x 160
+    //   FP64   0.47 / 0.45 / 0.50 (0.49)  1.69 / 1.69 / 1.68 (1.78)  5.62 / 5.39 / 4.41 (5.55)  1.28 / 1.34 / 1.24 (1.42)
+    //   FP32   0.35 / 0.34 / 0.36         1.20 / 1.27 / 1.30         4.24 / 3.98 / 3.37         1.02 / 1.01 / 0.94
+    constexpr int MINB = sizeof(T) == 4 ? 8 : 5;
+    if (b.nx >= 96) launch_as<T, MESH, RESP, PML, UP, false, MINB>(b, c, a);
+    else launch_as<T, MESH, RESP, PML, UP, true, MINB>(b, c, a);
+  } else if constexpr (MESH == MESH_CART || UP || (sizeof(T) == 4 ? RESP == RESP_EL : RESP != RESP_FQ8 || !PML)) {
+    // (the curvilinear blocks this leaves out run k_curv_fused: point_stage_ok)
     // The other elastic blocks and FP32 take the flattened points with 6 resident
     // CTAs (FP64 ms per step 0.56 flattened / 0.68 by the warp map on
     // 83 x 121 x 67 curvilinear points).  FP32 with at most 4 mechanisms has room
@@ -38,8 +49,11 @@ static void launch_point(Blk<T> &b, const StageCtx &c, const StageArgs &a) {
     // want the registers of 4 CTAs and no boundary columns among a warp's central
     // ones: 22.8 by the map / 23.4 flattened on the two-block Q8 hill of 201^3
     // points (27.7 with 6 CTAs), 1.57 / 1.77 on Q4 with PML of 93 x 118 x 75.
+    // fQ8 on a curvilinear block spills 236 bytes at 4 CTAs, none at 3: 2.79 ms
+    // per step against 3.13 on 101^3 (k_curv_fused 2.95).
     constexpr bool FLAT = sizeof(T) == 4 || RESP == RESP_EL;
-    constexpr int MINB = !FLAT ? 4 : sizeof(T) == 4 && (RESP == RESP_EL || RESP == RESP_Q4) ? 8 : 6;
+    constexpr int MINB = !FLAT ? (RESP == RESP_FQ8 && MESH == MESH_CURV && !UP ? 3 : 4)
+                               : sizeof(T) == 4 && (RESP == RESP_EL || RESP == RESP_Q4) ? 8 : 6;
     launch_as<T, MESH, RESP, PML, UP, FLAT, MINB>(b, c, a);
   }
 }
@@ -105,14 +119,36 @@ static bool tiles_faster(const Blk<T> &b) {
   return true;
 }
 
+// The curvilinear blocks that k_curv_fused is the faster kernel for (ms per
+// step, fused / point kernels).
+//  * FP32 with memory variables: both roles' code beside the 96 memory-variable
+//    streams outgrows the instruction cache; 6.27 / 6.55 on the hill of 145^3.
+//  * FP64 fQ8 with PML: 1.84 / 1.94 on 81^3, 5.26 / 5.30 on 121^3, with the
+//    registers of 3 CTAs (4 spill: 2.10, 5.73).
+//  * Small blocks with PML, whose third launch (k_pml_velocity) shows.  FP64
+//    elastic up to 2^16 points: 0.130 / 0.150 on 17^3, 0.140 / 0.147 on 33^3,
+//    0.208 / 0.179 on 41^3.  FP64 Q4 and Q8 from 2^14 to 2^16: 0.161 / 0.147 and
+//    0.171 / 0.161 on 25^3, 0.164 / 0.207 and 0.217 / 0.252 on 36^3, 0.278 /
+//    0.253 and 0.370 / 0.333 on 41^3.  FP32 elastic up to 1.2 million points:
+//    0.144 / 0.161 on 41^3, 1.20 / 1.27 on 101^3, 1.98 / 1.83 on 121^3.
+//    Not where a second block's kernels fill the gaps: two FP64 elastic blocks
+//    of 41 x 63 x 57 points 0.76 / 0.63, FP32 0.61 / 0.51.
+template <typename T>
+static bool fused_faster(const Blk<T> &b, int response, bool alone) {
+  bool pml = false;
+  for (int f = 0; f < 6; ++f) pml = pml || b.pml_on[f];
+  const long long n = (long long)b.nx * b.ny * b.nz;
+  if (sizeof(T) == 4) return b.nmech > 0 || (pml && alone && n < 1200000);
+  if (!pml) return false;
+  if (response == RESP_FQ8) return true;
+  return alone && n < (1 << 16) && (b.nmech == 0 || n >= (1 << 14));
+}
+
 // The point kernels keep one PML slab per axis: blocks whose two slabs on an
 // axis overlap (2 npml > n) take the generic passes.  Cartesian blocks need a
-// separable metric.  FP32 curvilinear blocks with memory variables stay with
-// k_curv_fused: 6.27 against 6.55 ms per step on the hill of 145^3 points
-// (both roles' code beside the 96 memory-variable streams outgrows the
-// instruction cache there).
+// separable metric.  alone: the domain's only block.
 template <typename T>
-bool point_stage_ok(const Blk<T> &b, int mesh) {
+bool point_stage_ok(const Blk<T> &b, int mesh, int response, bool alone) {
   const int nax[3] = {b.nx, b.ny, b.nz};
   for (int ax = 0; ax < 3; ++ax)
     if (b.pml_on[2 * ax] && b.pml_on[2 * ax + 1] && 2 * b.npml > nax[ax]) return false;
@@ -121,7 +157,7 @@ bool point_stage_ok(const Blk<T> &b, int mesh) {
       if (b.pml_on[f]) return false;   // upwind blocks with PML: the generic kernel
   }
   if (mesh == MESH_CART) return tuning().point && b.sep && (b.fd != 0 || !tiles_faster(b));
-  return tuning().curv_fused && tuning().lean && !(sizeof(T) == 4 && b.nmech > 0 && b.fd == 0);
+  return tuning().curv_fused && tuning().lean && (b.fd != 0 || !fused_faster(b, response, alone));
 }
 
 template <typename T>
@@ -133,7 +169,7 @@ void launch_fluxes(const Blk<T> &b, const StageCtx &c, int cur, int z0, int z1) 
 
 template void launch_fluxes<WQL3D_REAL>(const Blk<WQL3D_REAL> &, const StageCtx &, int, int, int);
 template void launch_point_stage<WQL3D_REAL>(Blk<WQL3D_REAL> &, int, const StageCtx &, const StageArgs &);
-template bool point_stage_ok<WQL3D_REAL>(const Blk<WQL3D_REAL> &, int);
+template bool point_stage_ok<WQL3D_REAL>(const Blk<WQL3D_REAL> &, int, int, bool);
 int WQL3D_CAT(upload_tables_point_, WQL3D_TAG)(const ConstTables &t) { return upload_tables_here(t); }
 
 }  // namespace wql3d

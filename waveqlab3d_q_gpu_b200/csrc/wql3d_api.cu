@@ -1017,7 +1017,7 @@ int setup_block(wql3d_domain *d, int bi) {
 template <typename T>
 bool point_path(wql3d_domain *d, int bi) {
   const Blk<T> &b = blk<T>(d, bi);
-  return !tuning().generic && !b.mms && point_stage_ok(b, d->hb[bi].mesh);
+  return !tuning().generic && !b.mms && point_stage_ok(b, d->hb[bi].mesh, d->response, d->nblocks == 1);
 }
 
 // the flux arrays of a curvilinear block on the point path, made current

@@ -97,8 +97,9 @@ void launch_point_stage(Blk<T> &b, int mesh, const StageCtx &c, const StageArgs 
 // blocks; the point kernels read them and leave the next stage's)
 template <typename T>
 void launch_fluxes(const Blk<T> &b, const StageCtx &c, int cur, int z0, int z1);
+// whether full stages of a block take the point kernels; alone: the domain's only block
 template <typename T>
-bool point_stage_ok(const Blk<T> &b, int mesh);
+bool point_stage_ok(const Blk<T> &b, int mesh, int response, bool alone);
 // true when the block's full curvilinear stages are one pass (k_curv_fused or
 // the point kernels, which can record the adjoint's derivative terms,
 // StageArgs::rec)
