@@ -376,9 +376,10 @@ int wql3d_get_adjoint_gradient(wql3d_domain *d, int block, double *g_material, d
    lists assign every CTA to one shot (128 points of one role of the point
    kernels; blocks with a full metric, and FP32 elastic shots above 2^20 points
    that are most of a batch: interior tiles and 128-point chunks of the
-   near-boundary shell).  The first run tunes the launch shape over its
-   first steps (each candidate times one step; the arithmetic of a point does
-   not depend on it) and keeps the fastest.  The batch orders
+   near-boundary shell).  The batch's first steps tune the launch shape
+   (each candidate times one step; the arithmetic of a point does not depend on
+   it); the fastest is kept, of those tried so far while runs were too short for
+   all.  The batch orders
    its work after the shots' own queued work and theirs after the batch; the
    shots' domains stay usable for set/get calls.  Domains must outlive the
    batch. */

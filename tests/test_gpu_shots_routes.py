@@ -38,3 +38,29 @@ def test_fp32_elastic_tiles_above_2_20_points(wql3d_lib):
         assert rel_l2(d.fields(0)[:3], F[:3]) < 1e-5
         assert rel_l2(d.fields(0)[3:], F[3:]) < 1e-5
     b.close()
+
+
+def test_tuner_goes_on_over_short_runs(wql3d_lib):
+    """A first run of one step keeps the shape to begin with (6 CTAs per SM in
+    FP64); the runs after it try all six, and the fastest of those tried is in
+    use.  The shape does not enter the arithmetic: one run of as many steps gives
+    the same fields to rounding of the contraction (1e-14 as in the other batch
+    test)."""
+    from waveqlab3d_q_gpu_b200.shots import ShotBatch, random_shots
+    ps = random_shots(3, nmin=21, nmax=33, steps=40)
+    a, b = ShotBatch(ps, nsteps_hint=13), ShotBatch(ps, nsteps_hint=13)
+    tried = []
+    for steps in (1, 2, 10):
+        a.run(steps)
+        shape, log = a.tuning()
+        tried.append(len(log))
+        assert len({c for c, _ in log}) == len(log)
+        assert shape == (min(log, key=lambda e: e[1])[0] if log else 6)
+        if steps == 1:
+            assert shape == 6
+    assert tried[0] <= 1 and tried[0] < tried[1] <= 3 and tried[2] == 6
+    b.run(13)
+    for d, e in zip(a.domains, b.domains):
+        assert rel_l2(d.fields(0), e.fields(0)) < 1e-14
+    a.close()
+    b.close()

@@ -2152,13 +2152,13 @@ struct wql3d_batch {
   int zchunk = 12;
   int minb = 6;                   // resident CTAs of the point kernels (FP32: 8 to begin with)
   bool points = false;            // every class runs the point kernels: minb is tuned, else zchunk
-  int tuned = 0;
+  int tuned = 0;                  // launch shapes tried so far
   int cur = 0;
   cudaGraphExec_t graph = nullptr;
   double g_dt = 0.0;
   int g_w = -1, g_cur = -1, g_z = -1, g_minb = -1;
   int64_t g_launches = 0, launches = 0;
-  std::vector<std::pair<int, float>> tune_log;   // (zchunk, ms per step) of the tuning steps
+  std::vector<std::pair<int, float>> tune_log;   // (launch shape, ms per step) of the tuning steps
 };
 
 namespace {
@@ -2223,18 +2223,18 @@ void batch_enqueue_step(wql3d_batch *bt, double dt, int w_stride) {
 
 template <typename T>
 int batch_run(wql3d_batch *bt, double dt, int nsteps, int w_stride) {
-  // project-written autotuner: the first steps of the first run each try one
-  // launch shape (the arithmetic of a point does not depend on it), timed with
-  // events; the fastest is kept: the resident CTAs of the point kernels, or the
-  // z-chunk length of the interior tiles where a shot needs those
-  if (!bt->tuned) {
-    const int zcand[6] = {4, 8, 12, 16, 24, 32}, pcand[6] = {3, 4, 5, 6, 7, 8};
-    const int *cand = bt->points ? pcand : zcand;
+  // project-written autotuner: the batch's first steps each try one launch
+  // shape (the arithmetic of a point does not depend on it), timed with events;
+  // the fastest is kept: the resident CTAs of the point kernels, or the z-chunk
+  // length of the interior tiles where a shot needs those.  A run too short to
+  // try them all leaves the rest to the next one and the fastest so far in use,
+  // so the first is the one that is right most often.
+  if (bt->tuned < 6 && nsteps > 0) {
+    static const int zcand[6] = {12, 16, 8, 24, 4, 32}, p64[6] = {6, 5, 4, 7, 8, 3}, p32[6] = {8, 7, 6, 5, 4, 3};
+    const int *cand = !bt->points ? zcand : bt->fp32 ? p32 : p64;
     int &shape = bt->points ? bt->minb : bt->zchunk;
-    float best = 1e30f;
-    int bestz = shape;
-    for (int i = 0; i < 6 && nsteps > 0; ++i) {
-      shape = cand[i];
+    for (; bt->tuned < 6 && nsteps > 0; ++bt->tuned, --nsteps) {
+      shape = cand[bt->tuned];
       if (int rc = batch_tiles(bt)) return rc;
       cudaEvent_t e0, e1;
       CK(cudaEventCreate(&e0));
@@ -2247,13 +2247,12 @@ int batch_run(wql3d_batch *bt, double dt, int nsteps, int w_stride) {
       CK(cudaEventElapsedTime(&ms, e0, e1));
       cudaEventDestroy(e0);
       cudaEventDestroy(e1);
-      bt->tune_log.push_back({cand[i], ms});
-      if (ms < best) { best = ms; bestz = cand[i]; }
-      --nsteps;
+      bt->tune_log.push_back({shape, ms});
     }
-    shape = bestz;
+    const auto best = std::min_element(bt->tune_log.begin(), bt->tune_log.end(),
+                                       [](const auto &p, const auto &q) { return p.second < q.second; });
+    shape = best->first;
     if (int rc = batch_tiles(bt)) return rc;
-    bt->tuned = 1;
   }
   // CUDA graph of two steps of the whole batch, replayed
   const int pairs = nsteps / 2;
