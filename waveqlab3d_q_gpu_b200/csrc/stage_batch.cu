@@ -122,6 +122,19 @@ __global__ void k_batch_advance(DevTime *const *times, int n, double dt) {
   tm->n = tm->n + 1;
 }
 
+// the point kernel compiled for minb resident CTAs (3 to 8)
+template <typename T, int RESP>
+auto point_kernel(int minb) {
+  switch (minb) {
+    case 3: return k_batch_point<T, RESP, 3>;
+    case 4: return k_batch_point<T, RESP, 4>;
+    case 5: return k_batch_point<T, RESP, 5>;
+    case 7: return k_batch_point<T, RESP, 7>;
+    case 8: return k_batch_point<T, RESP, 8>;
+    default: return k_batch_point<T, RESP, 6>;
+  }
+}
+
 // interior tiles (part 0) or near-boundary shell (part 1) of one class
 template <typename T, int RESP>
 void launch_class(const BatchClass<T> &C, const StageArgs &a, int zchunk, int minb, cudaStream_t s, int part,
@@ -130,14 +143,7 @@ void launch_class(const BatchClass<T> &C, const StageArgs &a, int zchunk, int mi
     if (part != 0 || C.tiles <= 0) return;
     StageArgs la = a;
     la.pf = sizeof(T) == 4 ? 1 : 0;
-    switch (minb) {
-      case 3: k_batch_point<T, RESP, 3><<<C.tiles, 128, 0, s>>>(C, la); break;
-      case 4: k_batch_point<T, RESP, 4><<<C.tiles, 128, 0, s>>>(C, la); break;
-      case 5: k_batch_point<T, RESP, 5><<<C.tiles, 128, 0, s>>>(C, la); break;
-      case 7: k_batch_point<T, RESP, 7><<<C.tiles, 128, 0, s>>>(C, la); break;
-      case 8: k_batch_point<T, RESP, 8><<<C.tiles, 128, 0, s>>>(C, la); break;
-      default: k_batch_point<T, RESP, 6><<<C.tiles, 128, 0, s>>>(C, la); break;
-    }
+    point_kernel<T, RESP>(minb)<<<C.tiles, 128, 0, s>>>(C, la);
     ++*launches;
     return;
   }
@@ -171,7 +177,23 @@ void launch_part(const BatchClass<T> *classes, int ncls, const StageArgs &a, int
   }
 }
 
+template <typename T, int RESP>
+void load_points() {
+  cudaFuncAttributes at;
+  for (int m = 3; m <= 8; ++m) cudaFuncGetAttributes(&at, point_kernel<T, RESP>(m));
+}
+
 }  // namespace
+
+template <typename T>
+void load_batch_point_kernels(int resp) {
+  switch (resp) {
+    case RESP_EL: load_points<T, RESP_EL>(); break;
+    case RESP_Q4: load_points<T, RESP_Q4>(); break;
+    case RESP_Q8: load_points<T, RESP_Q8>(); break;
+    default: load_points<T, RESP_FQ8>(); break;
+  }
+}
 
 // Shots whose tile kernel is faster than the point kernels where they make up
 // the batch: FP32 elastic above 2^20 points.  ms per step, tiles beside the
@@ -215,6 +237,7 @@ void launch_batch_advance(DevTime *const *times, int nshots, double dt, cudaStre
   ++*launches;
 }
 
+template void load_batch_point_kernels<WQL3D_REAL>(int);
 template bool batch_tiles_faster<WQL3D_REAL>(const Blk<WQL3D_REAL> &);
 template void launch_batch_stage<WQL3D_REAL>(const BatchClass<WQL3D_REAL> *, int, const StageArgs &, int,
                                              int, cudaStream_t, cudaStream_t, cudaEvent_t, cudaEvent_t, int64_t *);

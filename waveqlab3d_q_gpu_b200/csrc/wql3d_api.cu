@@ -2152,6 +2152,7 @@ struct wql3d_batch {
   int zchunk = 12;
   int minb = 6;                   // resident CTAs of the point kernels (FP32: 8 to begin with)
   bool points = false;            // every class runs the point kernels: minb is tuned, else zchunk
+  bool started = false;           // the first step is done
   int tuned = 0;                  // launch shapes tried so far
   int cur = 0;
   cudaGraphExec_t graph = nullptr;
@@ -2228,7 +2229,18 @@ int batch_run(wql3d_batch *bt, double dt, int nsteps, int w_stride) {
   // the fastest is kept: the resident CTAs of the point kernels, or the z-chunk
   // length of the interior tiles where a shot needs those.  A run too short to
   // try them all leaves the rest to the next one and the fastest so far in use,
-  // so the first is the one that is right most often.
+  // so the first is the one that is right most often.  No step that is timed
+  // pays for a first use: every candidate's kernel is loaded beforehand (half a
+  // step's time each on shots of 21 to 33 points an axis), and the batch's first
+  // step, in the shape to begin with, is not timed (its fields are not in L2 and
+  // the sample, advance and tile kernels load in it).
+  if (!bt->started) {
+    for (const auto &c : bt->cls)
+      if (bt->points && !c.shots.empty()) load_batch_point_kernels<T>(c.resp);
+    batch_enqueue_step<T>(bt, dt, w_stride);
+    bt->started = true;
+    --nsteps;
+  }
   if (bt->tuned < 6 && nsteps > 0) {
     static const int zcand[6] = {12, 16, 8, 24, 4, 32}, p64[6] = {6, 5, 4, 7, 8, 3}, p32[6] = {8, 7, 6, 5, 4, 3};
     const int *cand = !bt->points ? zcand : bt->fp32 ? p32 : p64;

@@ -21,6 +21,9 @@ struct BatchClass {
   DevTime *const *times;   // every shot's step time / sample counter (device)
 };
 
+// loads every point kernel of a response (a kernel is loaded at its first use otherwise)
+template <typename T>
+void load_batch_point_kernels(int resp);
 template <typename T>
 bool batch_tiles_faster(const Blk<T> &b);
 // zchunk: planes of an interior tile; minb: resident CTAs the point kernels
