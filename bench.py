@@ -576,9 +576,10 @@ def adjoint_leg(args, barrier):
 
 
 def shots_main(args, rank, world, local, barrier, max_over_ranks):
-    """Batched shots: every shot a domain on its own stream, replayed
-    round-robin; the timed region spans all streams (each stream's end event
-    joins the first stream before the stop event)."""
+    """Batched shots: one launch per kernel kind and stage for all shots, and for
+    comparison every shot a domain on its own stream, replayed round-robin; the
+    timed region spans all streams (each stream's end event joins the first
+    stream before the stop event)."""
     import numpy as np
     import torch
     from waveqlab3d_q_gpu_b200.shots import ShotBatch, random_shots
@@ -612,7 +613,7 @@ def shots_main(args, rank, world, local, barrier, max_over_ranks):
     for prec in ("fp32", "fp64", "fp32-streams"):
         mode = "streams" if prec.endswith("streams") else "batched"
         batch = ShotBatch(ps, precision=prec[:4], nsteps_hint=W + 2 * K + 10, mode=mode)
-        batch.run(max(W, 8))           # warm-up; the batched mode's tile autotuner uses its first 6 steps
+        batch.run(max(W, 8))           # warm-up; the batched mode's autotuner uses its first 7 steps
         batch.synchronize()
         l0 = batch.kernel_launches()
         clocks = ClockSampler(local) if prec == "fp32" else None
@@ -675,13 +676,15 @@ def shots_main(args, rank, world, local, barrier, max_over_ranks):
                 "e2e": e2e, "gpu_launches": r["launches"],
                 "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                              "frac": achieved / peak, "traffic": None, "peak_kind": peak_kind,
-                             "kernel": "whole step of every shot (stage kernels, concurrent streams)",
+                             "kernel": "whole step of every shot (batched stage kernels)",
                              "alg_bytes_per_step": words * 4 * 5},
                 "cpu_baseline": cpu, "clocks": clk,
                 "fp64": {"value": res["fp64"]["value"], "ms_per_step": res["fp64"]["ms"] / K},
-                "batched": {"launches_per_step": r["launches"] / K, "zchunk": r["tuning"][0],
+                "batched": {"launches_per_step": r["launches"] / K, "launch_shape": r["tuning"][0],
                             "tuning_ms_per_step": {str(z): m for z, m in r["tuning"][1]},
-                            "what": "one launch per kernel kind and RK stage for all shots, two-step CUDA graph"},
+                            "what": "one launch per kernel kind and RK stage for all shots, two-step CUDA graph; "
+                                    "launch_shape and the keys of tuning_ms_per_step: CTAs per SM of the point kernels, "
+                                    "or planes per interior tile where a class of shots runs the tiles"},
                 "streams": {"value": res["fp32-streams"]["value"], "ms_per_step": res["fp32-streams"]["ms"] / K,
                             "launches_per_step": res["fp32-streams"]["launches"] / K,
                             "what": "each shot its own stream and step graph, replayed round-robin"},
