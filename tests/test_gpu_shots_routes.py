@@ -44,6 +44,68 @@ def test_fp32_elastic_tiles_above_2_20_points(wql3d_lib):
     b.close()
 
 
+def _shot(seed, n, response, literal=False):
+    import numpy as np
+    from waveqlab3d_q_gpu_b200.shots import random_shot
+    p = random_shot(seed, n, n + 9, steps=NSTEPS + 2, response="elastic" if response == "anelastic-fQ8" else response)
+    if response == "anelastic-fQ8":
+        p.response = response
+        p.anelastic.tau = list(np.exp(np.linspace(np.log(0.008), np.log(3.0), 8)))
+        p.anelastic.strength_s = list(0.004 + 0.001 * np.arange(8))
+        p.anelastic.strength_p = list(0.002 + 0.0007 * np.arange(8))
+    p.closure_f32_literal = literal
+    return p
+
+
+CLASSES = {   # (response, full metric) of each shot
+    "separable": [("elastic", False), ("anelastic-Q4", False), ("elastic", False)],
+    "full metric": [("elastic", True), ("anelastic-Q4", True), ("elastic", True)],
+    "mixed": [("elastic", False), ("elastic", True), ("anelastic-Q4", False), ("anelastic-Q4", True)],
+    "Q8": [("anelastic-Q8", False), ("anelastic-Q8", True)],
+    "fQ8": [("anelastic-fQ8", False), ("anelastic-fQ8", True)],
+}
+
+
+@pytest.mark.parametrize("name", sorted(CLASSES))
+def test_every_route_equals_single_runs(wql3d_lib, oracle_lib, name):
+    """FP64: the batched kernels inline the bodies of the single-run ones, with the
+    descriptor in shared memory, so only the contraction of products may differ:
+    60 stages of a few roundings of 1.1e-16 stay below 1e-13.  One shot of each
+    route against the oracle at 1e-11, as in the other run tests."""
+    from waveqlab3d_q_gpu_b200.shots import ShotBatch
+    shots = CLASSES[name]
+    ps = [_shot(70 + i, 21, r, lit) for i, (r, lit) in enumerate(shots)]
+    b = ShotBatch(ps, nsteps_hint=NSTEPS)
+    b.run(NSTEPS)
+    b.synchronize()
+    classes = set(shots)
+    assert b.kernel_launches() == NSTEPS * (2 + 5 * sum(2 if lit else 1 for _, lit in classes))
+    for i, (p, d) in enumerate(zip(ps, b.domains)):
+        F, s = _single(p)
+        assert abs(F).max() > 0
+        assert rel_l2(d.fields(0), F) < 1e-13
+        assert rel_l2(d.seismograms(0)[:, :, 1:], s[:, :, 1:]) < 1e-13
+        if shots[i] not in shots[:i]:
+            o = oracle_lib.OracleDomain(p)
+            o.run(NSTEPS)
+            assert rel_l2(d.fields(0), o.fields(0)) < 1e-11
+    b.close()
+
+
+@pytest.mark.parametrize("name", ["Q8", "fQ8"])
+def test_fp32_memory_variables_in_a_batch(wql3d_lib, name):
+    """FP32 within 1e-5 of FP64 over 12 steps, as in the other FP32-batch test."""
+    from waveqlab3d_q_gpu_b200.shots import ShotBatch
+    ps = [_shot(70 + i, 21, r, lit) for i, (r, lit) in enumerate(CLASSES[name])]
+    b = ShotBatch(ps, precision="fp32", nsteps_hint=NSTEPS)
+    b.run(NSTEPS)
+    for p, d in zip(ps, b.domains):
+        F, _ = _single(p)
+        assert rel_l2(d.fields(0)[:3], F[:3]) < 1e-5
+        assert rel_l2(d.fields(0)[3:], F[3:]) < 1e-5
+    b.close()
+
+
 def test_tuner_goes_on_over_short_runs(wql3d_lib):
     """A first run of one step keeps the shape to begin with (6 CTAs per SM in
     FP64); the runs after it try all six, and the fastest of those tried is in
