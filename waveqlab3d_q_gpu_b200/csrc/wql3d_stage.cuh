@@ -46,7 +46,7 @@ struct Tuning {
   int mvpf = -1;      // k_curv_fused: L2 prefetch of the memory variables on entry (-1: FP32 only)
   int overlap = 1;    // side stream in use: the shell beside the interior tiles, the second block's point kernels beside
                       // the first's (0: every stage on one stream)
-  int point = 1;      // separable Cartesian stages through the point kernels (0 when WQL3D_TMA is set: the tile kernel)
+  int point = 1;      // separable Cartesian stages through the point kernels (0 when WQL3D_TMA has a value: the tile kernel)
   int tma = 0;        // Cartesian interior: 1 = planes filled by TMA box loads (default: cp.async, measured faster);
                       // 2 = TMA waits with no copies issued (test of the bounded waits and the stall status)
 };
@@ -58,8 +58,9 @@ inline Tuning tuning() {
     if (const char *e = getenv("WQL3D_FUSED_MINB")) r.fused_minb = atoi(e);
     if (const char *e = getenv("WQL3D_MV_PREFETCH")) r.mvpf = atoi(e);
     if (const char *e = getenv("WQL3D_SHELL_OVERLAP")) r.overlap = atoi(e);
-    if (const char *e = getenv("WQL3D_TMA")) {
-      r.tma = atoi(e);
+    const char *tma = getenv("WQL3D_TMA");
+    if (tma && *tma) {
+      r.tma = atoi(tma);
       r.point = 0;
     }
     if (const char *e = getenv("WQL3D_KERNEL")) {
