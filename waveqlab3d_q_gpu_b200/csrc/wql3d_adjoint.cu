@@ -27,8 +27,8 @@ __global__ void __launch_bounds__(128, REC ? 5 : 3) k_adj_pre(const __grid_const
   if (!flat_point(b, x, y, z)) return;
   const long long p = pidx(b, x, y, z);
   const long long V = b.vol;
-  // R is kept in memory only where a later pass of the stage reads it: the
-  // face points (k_adj_face) and the sources' support box (k_adj_moment)
+  // R is kept in memory only where a later pass of the stage reads it
+  // (k_adj_face): the face points and the sources' support box
   const bool keepR = x == 1 || x == b.nx || y == 1 || y == b.ny || z == 1 || z == b.nz ||
                      (x >= b.sbox[0] && x <= b.sbox[1] && y >= b.sbox[2] && y <= b.sbox[3] && z >= b.sbox[4] &&
                       z <= b.sbox[5]);

@@ -1840,10 +1840,12 @@ void transposed_rows(int n, int lit, std::vector<int> &off, std::vector<double> 
 }
 
 // recorded steps carry the stage inputs' derivative terms when the block's
-// stages run the fused curvilinear kernel (the Cartesian kernels do not write
-// them; the adjoint then recomputes them)
+// stages run one of the curvilinear one-pass kernels, which write them (the
+// point kernels, or k_curv_fused); where they do not, the adjoint recomputes them
 bool record_terms(wql3d_domain *d) {
-  return d->hb[0].mesh == WQL3D_MESH_CURVILINEAR && !tuning().generic && curv_stage_fused(d->bd[0]);
+  const Blk<double> &b = d->bd[0];
+  if (d->hb[0].mesh != WQL3D_MESH_CURVILINEAR || tuning().generic || b.mms) return false;
+  return b.fd == WQL3D_FD_TRADITIONAL6 ? curv_stage_fused(b) : point_path<double>(d, 0);
 }
 
 int adjoint_supported(wql3d_domain *d) {
@@ -1949,8 +1951,8 @@ int wql3d_record_step(wql3d_domain *d, double dt, int n, int w_stride, double *d
   h.n = n;
   CK(cudaMemcpyAsync(d->time, &h, sizeof(h), cudaMemcpyHostToDevice, d->stream));
   if (int rc = enqueue_sample<double>(d, w_stride)) return rc;
-  // stage inputs, then (blocks on the fused curvilinear kernel) the stage
-  // inputs' derivative terms written by the stage kernel itself
+  // stage inputs, then (record_terms) the stage inputs' derivative terms
+  // written by the stage kernel itself
   const bool terms = record_terms(d);
   for (int s = 1; s <= 5; ++s) {
     CK(cudaMemcpyAsync(dev_out + (s - 1) * ne, d->cur ? b.F1 : b.F0, sizeof(double) * ne, cudaMemcpyDeviceToDevice,

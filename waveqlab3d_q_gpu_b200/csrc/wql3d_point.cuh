@@ -270,7 +270,7 @@ __device__ __forceinline__ void face_term(const Blk<T> &b, const T *__restrict__
 
 // PML slab and physical boundary of axis AX for this role's components: G
 // holds the axis' three source terms (fluxes over J, or velocity gradients)
-template <int AX, typename T, int MESH, int ROLE, bool PML, bool FACE = true>
+template <int AX, typename T, int MESH, int ROLE, bool PML>
 __device__ __forceinline__ void axis_finish(const Blk<T> &b, const StageArgs &a, const T *__restrict__ F, int x, int y,
                                             int z, long long p, const T G[3], T irho, T l2m, T lam, T mu,
                                             T df[RoleComps<ROLE>::N], T e[6]) {
@@ -280,7 +280,7 @@ __device__ __forceinline__ void axis_finish(const Blk<T> &b, const StageArgs &a,
   const int n = axis_len<AX>(b);
   T dq[NC];
   const int f = i == 1 ? 2 * AX : i == n ? 2 * AX + 1 : -1;
-  const bool sat = FACE && f >= 0 && b.bc[f] > 0;
+  const bool sat = f >= 0 && b.bc[f] > 0;
   if (sat) {
     T ds[NC];
     face_term<AX, T, MESH, ROLE>(b, F, f, x, y, z, p, ds, dq);
@@ -300,44 +300,44 @@ __device__ __forceinline__ void axis_finish(const Blk<T> &b, const StageArgs &a,
         // the auxiliary velocities themselves: k_pml_velocity
 #pragma unroll
         for (int c = 0; c < 3; ++c) df[c] = df[c] - d * Qp[c * PV] * irho;
-        return;
-      }
-      T Q[NC], DQ[NC];
-#pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        Q[c] = Qp[c * PV];
-        DQ[c] = A * DQp[c * PV];
-      }
-      if constexpr (ROLE == ROLE_V) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          df[c] = df[c] - d * Q[c] * irho;
-          DQ[c] = DQ[c] + G[c] - (d + (T)1) * Q[c];
-        }
       } else {
-        df[0] = df[0] - d * (l2m * Q[0] + lam * Q[1] + lam * Q[2]);
-        df[1] = df[1] - d * (lam * Q[0] + l2m * Q[1] + lam * Q[2]);
-        df[2] = df[2] - d * (lam * Q[0] + lam * Q[1] + l2m * Q[2]);
+        T Q[NC], DQ[NC];
 #pragma unroll
-        for (int c = 3; c < 6; ++c) df[c] = df[c] - mu * d * Q[c];
-        // strain rates of the memory variables (src/RHS_Interior.f90:2351-2451)
-        e[C::c0 - 3] = e[C::c0 - 3] - d * Q[C::c0 - 3];
-        e[C::c1 - 3] = e[C::c1 - 3] - d * Q[C::c1 - 3];
-        e[C::c2 - 3] = e[C::c2 - 3] - d * Q[C::c2 - 3];
-#pragma unroll
-        for (int c = 0; c < 6; ++c) {
-          const T src = c == C::c0 - 3 ? G[0] : c == C::c1 - 3 ? G[1] : c == C::c2 - 3 ? G[2] : (T)0;
-          DQ[c] = DQ[c] + src - (d + (T)1) * Q[c];
+        for (int c = 0; c < NC; ++c) {
+          Q[c] = Qp[c * PV];
+          DQ[c] = A * DQp[c * PV];
         }
-      }
-      if (sat && s == f) {
+        if constexpr (ROLE == ROLE_V) {
 #pragma unroll
-        for (int c = 0; c < NC; ++c) DQ[c] = DQ[c] - dq[c];
-      }
+          for (int c = 0; c < 3; ++c) {
+            df[c] = df[c] - d * Q[c] * irho;
+            DQ[c] = DQ[c] + G[c] - (d + (T)1) * Q[c];
+          }
+        } else {
+          df[0] = df[0] - d * (l2m * Q[0] + lam * Q[1] + lam * Q[2]);
+          df[1] = df[1] - d * (lam * Q[0] + l2m * Q[1] + lam * Q[2]);
+          df[2] = df[2] - d * (lam * Q[0] + lam * Q[1] + l2m * Q[2]);
 #pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        DQp[c * PV] = DQ[c];
-        Qp[c * PV] = Q[c] + Bdt * DQ[c];
+          for (int c = 3; c < 6; ++c) df[c] = df[c] - mu * d * Q[c];
+          // strain rates of the memory variables (src/RHS_Interior.f90:2351-2451)
+          e[C::c0 - 3] = e[C::c0 - 3] - d * Q[C::c0 - 3];
+          e[C::c1 - 3] = e[C::c1 - 3] - d * Q[C::c1 - 3];
+          e[C::c2 - 3] = e[C::c2 - 3] - d * Q[C::c2 - 3];
+#pragma unroll
+          for (int c = 0; c < 6; ++c) {
+            const T src = c == C::c0 - 3 ? G[0] : c == C::c1 - 3 ? G[1] : c == C::c2 - 3 ? G[2] : (T)0;
+            DQ[c] = DQ[c] + src - (d + (T)1) * Q[c];
+          }
+        }
+        if (sat && s == f) {
+#pragma unroll
+          for (int c = 0; c < NC; ++c) DQ[c] = DQ[c] - dq[c];
+        }
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+          DQp[c * PV] = DQ[c];
+          Qp[c * PV] = Q[c] + Bdt * DQ[c];
+        }
       }
     }
   }
