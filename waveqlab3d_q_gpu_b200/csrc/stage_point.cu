@@ -121,8 +121,10 @@ static bool tiles_faster(const Blk<T> &b) {
 
 // The curvilinear blocks that k_curv_fused is the faster kernel for (ms per
 // step, fused / point kernels).
-//  * FP32 with memory variables: both roles' code beside the 96 memory-variable
-//    streams outgrows the instruction cache; 6.27 / 6.55 on the hill of 145^3.
+//  * FP32 with memory variables: 6.27 / 6.55 on the hill of 145^3 (likely both
+//    roles' code, beside 96 memory-variable streams, in the instruction cache).
+//    With an upwind pair the other path is the generic kernel: 3.61 / 1.17 on
+//    97 x 89 x 83 points, Q8, upwind-4.
 //  * FP64 fQ8 with PML: 1.84 / 1.94 on 81^3, 5.26 / 5.30 on 121^3, with the
 //    registers of 3 CTAs (4 spill: 2.10, 5.73).
 //  * Small blocks with PML, whose third launch (k_pml_velocity) shows.  FP64
