@@ -50,3 +50,29 @@ def test_row_lengths(wql3d_lib, oracle_lib, nx, pml):
 @pytest.mark.parametrize("n,launches", [((139, 139, 139), 2), ((139, 138, 140), 1)])
 def test_tiles_from_139_points_an_axis(wql3d_lib, oracle_lib, n, launches):
     assert _stages(oracle_lib, small_case(response="elastic", n=n), ("fp64",)) == launches
+
+
+def test_slabs_on_the_tiles_equal_the_whole_block(wql3d_lib):
+    """Two s-slabs of 139 planes: each runs the tiles, whose strict interior reaches
+    the open face.  Equal to the whole block to rounding, 1e-12 as in the other
+    slab tests."""
+    import numpy as np
+    from waveqlab3d_q_gpu_b200.domain import Domain
+    from waveqlab3d_q_gpu_b200.slabs import SlabSet
+    p = small_case(response="elastic", n=(139, 139, 278))
+    (F, _), = random_state(p, scale=1e-3)
+    g = Domain(p, nsteps_hint=4)
+    g.set_fields(F)
+    g.run(3)
+    ss = SlabSet(p, 2, nsteps_hint=4, cuts=(139, 139))
+    for part, d in zip(ss.parts, ss.domains):
+        d.set_fields(F[:, part.z0:part.z0 + 139])
+    before = ss.domains[0].kernel_launches()
+    ss.run(3)
+    # a step: sample, per stage two stage kernels, a halo pack and an unpack, advance
+    assert ss.domains[0].kernel_launches() - before == 3 * (2 + 5 * 4)
+    Fw = g.fields(0)
+    assert np.abs(Fw).max() > 0
+    assert rel_l2(ss.fields(), Fw) < 1e-12
+    ss.close()
+    g.close()

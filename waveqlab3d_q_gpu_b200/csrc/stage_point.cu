@@ -43,9 +43,10 @@ static void launch_point(Blk<T> &b, const StageCtx &c, const StageArgs &a) {
     // (the curvilinear blocks this leaves out run k_curv_fused: point_stage_ok)
     // The other elastic blocks and FP32 take the flattened points with 6 resident
     // CTAs (FP64 ms per step 0.56 flattened / 0.68 by the warp map on
-    // 83 x 121 x 67 curvilinear points).  FP32 with at most 4 mechanisms has room
-    // for 8 CTAs: 1.21 against 1.24 on Q4 with PML of 93 x 118 x 75 (fQ8: 7.06
-    // against 6.29 on 96 x 160 x 128 twice, so 6 there).  Memory variables in FP64
+    // 83 x 121 x 67 curvilinear points).  FP32 with at most 4 mechanisms runs
+    // with 8 CTAs, which spills 8 to 104 bytes and still gains: 1.21 against 1.24
+    // on Q4 with PML of 93 x 118 x 75 (fQ8: 7.06 against 6.29 on 96 x 160 x 128
+    // twice, so 6 there).  Memory variables in FP64
     // want the registers of 4 CTAs and no boundary columns among a warp's central
     // ones: 22.8 by the map / 23.4 flattened on the two-block Q8 hill of 201^3
     // points (27.7 with 6 CTAs), 1.57 / 1.77 on Q4 with PML of 93 x 118 x 75.
