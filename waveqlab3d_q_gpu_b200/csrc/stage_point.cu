@@ -107,17 +107,39 @@ void launch_point_stage(Blk<T> &b, int mesh, const StageCtx &c, const StageArgs 
   }
 }
 
-// FP64 elastic Cartesian blocks without PML whose shortest axis has 139 points
-// or more: the tile kernel beside the shell is the faster one there (ms per
-// step, tiles / point kernel: 137^3 1.55 / 1.53, 145 x 141 x 139 1.75 / 1.82, 160^3 2.29 /
-// 2.34, 201^3 4.14 / 4.22; a short axis makes the shell large: 200 x 200 x 90
-// 1.97 / 1.86, 160 x 160 x 31 0.66 / 0.50).
+// The elastic Cartesian blocks that the tile kernel beside the shell is the
+// faster one for (ms per step, tiles / point kernel).
+//  * FP64 without PML, shortest axis 139 points or more: 137^3 1.55 / 1.53,
+//    145 x 141 x 139 1.75 / 1.82, 160^3 2.29 / 2.34, 201^3 4.14 / 4.22; a short
+//    axis makes the shell large: 200 x 200 x 90 1.97 / 1.86, 160 x 160 x 31 0.66 /
+//    0.50.
+//  * FP64 with PML, little of it and little shell: the point kernel's PML form
+//    costs every point, the tiles' only the slabs.  Slabs of `layer` points on
+//    `faces` faces, shell (its share of the points) and slab share beside it:
+//      101^3          1 face of 5    .32  .05   0.94 / 1.04
+//      101^3          2 faces of 10  .38  .19   1.14 / 1.22
+//      101^3          3 faces of 10  .40  .27   1.24 / 1.25
+//      145^3          2 faces of 5   .23  .07   2.36 / 2.69
+//      145^3          3 faces of 10  .30  .19   2.84 / 2.80
+//      160^3          5 faces of 8   .26  .23   3.61 / 3.49
+//       81 x 79 x 83  1 face of 5    .38  .06   0.66 / 0.59
+//      short rows, flattened, lose at any slab share:
+//       70 x 160 x 160  3 faces of 10  .38  .25   1.90 / 2.19
+//  * FP32 with PML: 145^3 1 face of 5 (.23, .03) 2.00 / 2.08, 2 faces of 10
+//    (.27, .13) 2.33 / 2.16.
 template <typename T>
 static bool tiles_faster(const Blk<T> &b) {
-  if (sizeof(T) == 4 || b.nmech > 0 || b.nx < 139 || b.ny < 139 || b.nz < 139) return false;
-  for (int f = 0; f < 6; ++f)
-    if (b.pml_on[f]) return false;
-  return true;
+  if (b.nmech > 0) return false;
+  const int n[3] = {b.nx, b.ny, b.nz};
+  double inner = 1.0, clear = 1.0;
+  for (int ax = 0; ax < 3; ++ax) {
+    inner *= (double)(b.hi[ax] - b.lo[ax] + 1) / n[ax];
+    clear *= 1.0 - (double)b.npml * (b.pml_on[2 * ax] + b.pml_on[2 * ax + 1]) / n[ax];
+  }
+  const double shell = 1.0 - inner, slab = 1.0 - clear;
+  if (slab == 0.0) return sizeof(T) == 8 && b.nx >= 139 && b.ny >= 139 && b.nz >= 139;
+  if (sizeof(T) == 4) return shell < 0.24 && slab < 0.1;
+  return shell < 0.38 && (b.nx < 96 || slab < 0.2);
 }
 
 // The curvilinear blocks that k_curv_fused is the faster kernel for (ms per
