@@ -26,9 +26,12 @@ static void launch_point(Blk<T> &b, const StageCtx &c, const StageArgs &a) {
     //   FP32       0.31 / 0.36  0.56 / 0.58  1.41 / 1.29  2.12 / 1.94  1.89 / 1.66     2.00 / 2.10
     //   FP32, PML  0.55 / 0.57  1.04 / 1.00               3.63 / 2.69
     // FP64 flattened with 6 CTAs spills 136 bytes (272 with PML; 5 CTAs: none, 32):
-    // 0.70 at 101^3, 0.088 against 0.082 at 41^3.
+    // 0.70 at 101^3, 0.088 against 0.082 at 41^3.  A block that shares the GPU with
+    // the domain's other one gains from the sixth: two of 121 x 101 x 111 points
+    // 2.05 against 2.10, with PML two of 81 x 83 x 85 1.52 against 1.56.
     if (b.nx >= (PML ? 96 : 125)) launch_as<T, MESH, RESP, PML, UP, false, sizeof(T) == 4 ? 8 : 6>(b, c, a);
-    else launch_as<T, MESH, RESP, PML, UP, true, sizeof(T) == 4 ? 8 : 5>(b, c, a);
+    else if (c.alone) launch_as<T, MESH, RESP, PML, UP, true, sizeof(T) == 4 ? 8 : 5>(b, c, a);
+    else launch_as<T, MESH, RESP, PML, UP, true, sizeof(T) == 4 ? 8 : 6>(b, c, a);
   } else if constexpr (RESP == RESP_EL && MESH == MESH_CURV && PML) {
     // Elastic curvilinear blocks with PML: the same line at 96 points a row, FP64
     // with 5 resident CTAs (6 spill 32 to 40 bytes), FP32 with 8; ms per step,

@@ -1034,7 +1034,7 @@ template <typename T>
 void launch_stage(wql3d_domain *d, int bi, const StageArgs &a, bool fused = false, cudaStream_t stream = nullptr) {
   Blk<T> &b = blk<T>(d, bi);
   const int mesh = d->hb[bi].mesh;
-  StageCtx c{stream ? stream : d->stream, d->response, &d->launches, d->side, d->fork, d->join};
+  StageCtx c{stream ? stream : d->stream, d->response, &d->launches, d->side, d->fork, d->join, d->nblocks == 1};
   const bool special = tuning().generic || b.mms || b.fd != WQL3D_FD_TRADITIONAL6;
   if (a.flags == F_ALL && point_path<T>(d, bi)) {
     ensure_fluxes<T>(d, bi);

@@ -34,6 +34,7 @@ struct StageCtx {
   // points, read-only F)
   cudaStream_t side = nullptr;
   cudaEvent_t fork = nullptr, join = nullptr;
+  bool alone = true;  // the domain's only block (false: the other one's kernels may run at the same time)
 };
 
 // tuning switches read once per translation unit from the environment
